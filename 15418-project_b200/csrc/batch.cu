@@ -132,6 +132,7 @@ gpjb::BatchQueryLaunch query_launch_of(const gpj_batch *b) {
   // (written by the finalize kernel just before the query launch)
   q.status = reinterpret_cast<unsigned int *>(b->d_totals + gpjb::kTotError);
   q.record_counter = reinterpret_cast<unsigned long long *>(b->d_totals + gpjb::kTotRecordCounter);
+  q.expected_records = b->records;
   q.num_groups = int(b->groups.size());
   for (size_t g = 0; g < b->groups.size(); ++g) q.groups[g] = b->groups[g];
   return q;

@@ -75,9 +75,12 @@ struct BatchQueryLaunch {
   int32_t *out = nullptr;
   unsigned int *status = nullptr;  // kQueryStatusOverflow is OR-ed here (optional)
   unsigned int *file_status = nullptr;  // or into one word per file (optional, first)
-  // records are handed to warps 32 at a time from this counter, which the
-  // launch zeroes first (optional; without it each thread strides)
+  // records are handed to warps from this counter, which the launch zeroes
+  // first (optional; without it each warp strides)
   unsigned long long *record_counter = nullptr;
+  // about the number of records (0: unknown, many): chooses the lanes per
+  // record and bounds the grid; the results do not depend on it
+  uint64_t expected_records = 0;
   int num_groups = 0;
   BatchQueryGroup groups[kMaxBatchGroups];
 };

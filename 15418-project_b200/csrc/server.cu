@@ -1014,9 +1014,9 @@ struct gpj_server {
     if (e == cudaSuccess) e = cudaMemsetAsync(d_stat, 0, V * 4u, s0.stream);
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device);
-    const uint64_t blocks = (records + 127u) / 128u;
-    const int grid = int(std::max<uint64_t>(1, std::min<uint64_t>(blocks, uint64_t(sms) * 8u)));
-    if (e == cudaSuccess && records > 0) e = gpjb::batch_query_launch(ql, blob, grid, 128, s0.stream);
+    ql.expected_records = records;
+    if (e == cudaSuccess && records > 0)
+      e = gpjb::batch_query_launch(ql, blob, std::max(sms, 1) * 8, 128, s0.stream);
     b->refs = int(in_batch.size());
     qbatches.emplace(b, std::move(owned));
     uint64_t v = 0;
