@@ -120,42 +120,6 @@ __device__ Agg lookback(const IndexLaunch &P, uint32_t tile) {
   return agg_unpack(later);
 }
 
-// ----------------------------------------------------------------------------
-// Leveled bitmaps of one word.  Walks the open/close events of the word in
-// order; separators between two events share one depth.  Depth arithmetic is
-// signed char, as in sharemem/leveled-bitmaps-index.cu:270-300.
-// ----------------------------------------------------------------------------
-template <int LMAX>
-__device__ __forceinline__ void add_level(uint64_t (&lb)[LMAX], int d, uint64_t m) {
-  // levels >= L are computed but never stored; d outside [0, LMAX) matches none
-#pragma unroll
-  for (int l = 0; l < LMAX; ++l) lb[l] |= (d == l) ? m : 0ull;
-}
-
-template <int LMAX>
-__device__ __forceinline__ int leveled_word(uint64_t op, uint64_t cl,
-                                            uint64_t sp, int depth,
-                                            uint64_t (&lb)[LMAX]) {
-#pragma unroll
-  for (int l = 0; l < LMAX; ++l) lb[l] = 0;
-  uint64_t ev = op | cl;
-  int d = depth;
-  uint64_t acc = 0, done = 0;
-  while (ev) {  // branch-free body: lanes only differ in the trip count
-    const uint64_t bit = ev & (0 - ev);
-    const uint64_t below = bit - 1;
-    acc |= sp & below & ~done;
-    const bool open = (op & bit) != 0;
-    add_level<LMAX>(lb, d, open ? acc : (acc | bit));
-    d = int(int8_t(open ? d + 1 : d - 1));
-    acc = open ? bit : 0ull;
-    done = below | bit;
-    ev &= ev - 1;
-  }
-  add_level<LMAX>(lb, d, acc | (sp & ~done));
-  return d;
-}
-
 __device__ __forceinline__ uint64_t valid_mask(uint64_t w, uint64_t n) {
   const uint64_t base = w * 64u;
   if (base + 64u <= n) return ~0ull;
@@ -372,7 +336,9 @@ struct PipeSmem {
 // level, one 64-bit slot for each of the warp's 64 words; a lane only ever
 // touches the slots of its own two words.  Level LMAX is a sink for the
 // masks of depths that are not stored, so the walk writes without a branch.
-constexpr int kSharedLevels = 8;  // LMAX up to this stages in shared memory
+// Indexes of more than kSharedLevels levels take them in passes of as many
+// (kPasses).
+constexpr int kSharedLevels = 8;
 // Indexes of up to four levels can walk quarters with two or more bracket
 // events from a per-warp list (every lane takes one), the rest in the lane
 // that owns them (kList); otherwise every lane walks its own four quarters.
@@ -394,8 +360,7 @@ struct RowState {
   uint32_t pex, par0, dd_ex, nl_ex;
 };
 
-// The leveled-bitmap scratch follows the pipeline state (8-byte aligned);
-// kernels for more than kSharedLevels levels do not allocate it.
+// The leveled-bitmap scratch follows the pipeline state (16-byte aligned).
 template <int NT>
 __host__ __device__ constexpr size_t level_scratch_offset() {
   return (sizeof(PipeSmem<NT>) + 15u) & ~size_t(15);
@@ -837,7 +802,7 @@ __device__ __forceinline__ void leveled_lane(LevelScratch<NT, LMAX, kList> &ls, 
   }
 }
 
-template <int LMAX, int NT, bool kList>
+template <int LMAX, int NT, bool kList, bool kPasses>
 __device__ __forceinline__ void phase_b(const IndexLaunch &P, PipeSmem<NT> &sm,
                                         LevelScratch<NT, LMAX, kList> &ls, uint32_t k,
                                         const RowState &st) {
@@ -880,33 +845,47 @@ __device__ __forceinline__ void phase_b(const IndexLaunch &P, PipeSmem<NT> &sm,
     store2(S_tile - tm.lw_tile, lw0, W, S0, S1);
   }
   if (levels > 0) {
-    uint64_t lb0[LMAX], lb1[LMAX];
     const uint64_t O0 = st.op0 & ~S0, C0 = st.cl0 & ~S0, P0 = st.sp0 & ~S0;
     const uint64_t O1 = st.op1 & ~S1, C1 = st.cl1 & ~S1, P1 = st.sp1 & ~S1;
-    if constexpr (LMAX <= kSharedLevels) {
-      leveled_lane<LMAX, NT, kList>(ls, O0, C0, P0, O1, C1, P1, depth0, lb0, lb1);
-    } else {
-      const int depth1 = leveled_word<LMAX>(O0, C0, P0, depth0, lb0);
-      leveled_word<LMAX>(O1, C1, P1, depth1, lb1);
-    }
-    if (inside && (flags & kTileAllAligned) != 0) {
+    uint64_t lb0[LMAX], lb1[LMAX];
+    leveled_lane<LMAX, NT, kList>(ls, O0, C0, P0, O1, C1, P1, depth0, lb0, lb1);
+    for (int first = 0;;) {
+      // levels first .. first + LMAX - 1, held in lb0 and lb1
+      uint64_t *const row0 = LB_tile + uint64_t(first) * W;
+      if (inside && (flags & kTileAllAligned) != 0) {
 #pragma unroll
-      for (int l = 0; l < LMAX; ++l) {
-        if (l < levels)
-          *reinterpret_cast<ulonglong2 *>(LB_tile + uint64_t(l) * W + 2 * tid) =
-              make_ulonglong2(lb0[l], lb1[l]);
+        for (int l = 0; l < LMAX; ++l) {
+          if (first + l < levels)
+            *reinterpret_cast<ulonglong2 *>(row0 + uint64_t(l) * W + 2 * tid) =
+                make_ulonglong2(lb0[l], lb1[l]);
+        }
+      } else if (inside) {
+#pragma unroll
+        for (int l = 0; l < LMAX; ++l) {
+          if (first + l < levels)
+            put2(row0 + uint64_t(l) * W, ((flags >> (kTileLevelAligned + first + l)) & 1u) != 0,
+                 lb0[l], lb1[l]);
+        }
+      } else {
+#pragma unroll
+        for (int l = 0; l < LMAX; ++l) {
+          if (first + l < levels)
+            store2(row0 - tm.lw_tile + uint64_t(l) * W, lw0, W, lb0[l], lb1[l]);
+        }
       }
-    } else if (inside) {
+      if constexpr (!kPasses) break;
+      first += LMAX;
+      if (first >= levels) break;
+      // The next levels are walked only by warps where some lane's depth may
+      // reach them (depths of a lane stay within its start depth plus its
+      // opening and minus its closing brackets); records rarely nest that
+      // deep, and the others store zeros.
+      const int opens = popc64(O0) + popc64(O1), closes = popc64(C0) + popc64(C1);
+      if (__any_sync(0xFFFFFFFFu, depth0 + opens >= first || depth0 - closes < -128)) {
+        leveled_lane<LMAX, NT, kList>(ls, O0, C0, P0, O1, C1, P1, depth0 - first, lb0, lb1);
+      } else {
 #pragma unroll
-      for (int l = 0; l < LMAX; ++l) {
-        if (l < levels)
-          put2(LB_tile + uint64_t(l) * W, ((flags >> (kTileLevelAligned + l)) & 1u) != 0, lb0[l],
-               lb1[l]);
-      }
-    } else {
-#pragma unroll
-      for (int l = 0; l < LMAX; ++l) {
-        if (l < levels) store2(LB_tile - tm.lw_tile + uint64_t(l) * W, lw0, W, lb0[l], lb1[l]);
+        for (int l = 0; l < LMAX; ++l) lb0[l] = lb1[l] = 0ull;
       }
     }
   }
@@ -930,9 +909,9 @@ __device__ __forceinline__ void phase_b(const IndexLaunch &P, PipeSmem<NT> &sm,
 
 // LMAX: levels the kernel can store; kTma: tiles staged by TMA; NT: compute
 // threads; kList: the listed leveled walk; kLB: look-back descriptors per
-// lane.
-template <int LMAX, bool kTma, int NT, bool kList, int kLB>
-__global__ void __launch_bounds__(NT + 32, LMAX > 8 ? 1 : (NT <= 128 ? 4 : 2))
+// lane; kPasses: more than LMAX levels, in passes.
+template <int LMAX, bool kTma, int NT, bool kList, int kLB, bool kPasses>
+__global__ void __launch_bounds__(NT + 32, NT <= 128 ? 4 : 2)
     index_kernel(const __grid_constant__ CUtensorMap tmap, const IndexLaunch P) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // the 128-byte-swizzled TMA destinations need 1024-byte alignment
@@ -978,18 +957,17 @@ __global__ void __launch_bounds__(NT + 32, LMAX > 8 ? 1 : (NT <= 128 ? 4 : 2))
     if (stop) break;
     RowState cur;
     phase_a<LMAX, kTma, NT>(P, sm, s, k, cur);
-    if (k > 0) phase_b<LMAX, NT, kList>(P, sm, ls, k - 1, prev);
+    if (k > 0) phase_b<LMAX, NT, kList, kPasses>(P, sm, ls, k - 1, prev);
     prev = cur;
   }
   if (k > 0 && !*static_cast<volatile uint32_t *>(&sm.abort))
-    phase_b<LMAX, NT, kList>(P, sm, ls, k - 1, prev);
+    phase_b<LMAX, NT, kList, kPasses>(P, sm, ls, k - 1, prev);
 }
 
-template <int LMAX, bool kTma, int NT, bool kList, int kLB>
+template <int LMAX, bool kTma, int NT, bool kList, int kLB, bool kPasses>
 cudaError_t launch_kernel(const IndexLaunch &L, const CUtensorMap &map, cudaStream_t stream) {
-  auto kernel = index_kernel<LMAX, kTma, NT, kList, kLB>;
-  constexpr size_t smem = level_scratch_offset<NT>() +
-                          (LMAX <= kSharedLevels ? sizeof(LevelScratch<NT, LMAX, kList>) : 0) +
+  auto kernel = index_kernel<LMAX, kTma, NT, kList, kLB, kPasses>;
+  constexpr size_t smem = level_scratch_offset<NT>() + sizeof(LevelScratch<NT, LMAX, kList>) +
                           1024;  // + alignment slack
   static int grid_per_device[64] = {};
   int dev = 0;
@@ -1012,12 +990,12 @@ cudaError_t launch_kernel(const IndexLaunch &L, const CUtensorMap &map, cudaStre
   return cudaGetLastError();
 }
 
-template <int LMAX, int NT, bool kList, int kLB>
+template <int LMAX, int NT, bool kList, int kLB, bool kPasses = false>
 cudaError_t launch_tma(const IndexLaunch &L, const CUtensorMap *map, bool use_tma,
                        cudaStream_t stream) {
-  if (use_tma) return launch_kernel<LMAX, true, NT, kList, kLB>(L, *map, stream);
+  if (use_tma) return launch_kernel<LMAX, true, NT, kList, kLB, kPasses>(L, *map, stream);
   CUtensorMap dummy{};
-  return launch_kernel<LMAX, false, NT, kList, kLB>(L, dummy, stream);
+  return launch_kernel<LMAX, false, NT, kList, kLB, kPasses>(L, dummy, stream);
 }
 
 // The launch variant (IndexLaunch::variant) picks the walk and the look-back
@@ -1044,8 +1022,11 @@ cudaError_t launch_threads(const IndexLaunch &L, const CUtensorMap *map, bool us
   const int lv = L.num_levels;
   if (lv <= 2) return launch_levels<2, NT>(L, map, use_tma, stream);
   if (lv <= 4) return launch_levels<4, NT>(L, map, use_tma, stream);
-  if (lv <= 8) return launch_levels<8, NT>(L, map, use_tma, stream);
-  return launch_levels<kMaxLevels, NT>(L, map, use_tma, stream);
+  if (lv <= kSharedLevels) return launch_levels<kSharedLevels, NT>(L, map, use_tma, stream);
+  // 96 MiB of posts: 8 levels 81 us; in passes 12, 15 and 22 levels 103, 104
+  // and 111 us (191, 193 and 197 us in an instance that held 22 levels in
+  // registers and went over all of them at every bracket)
+  return launch_tma<kSharedLevels, NT, false, 1, true>(L, map, use_tma, stream);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
