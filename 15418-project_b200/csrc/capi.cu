@@ -764,9 +764,14 @@ int gpj_results_compact(gpj_ctx *ctx, const int32_t *d_results, uint64_t num_lin
     return fail(GPJ_ERR_INVALID_ARGUMENT, "null match buffer");
   if (num_result_slots > 0 && num_lines > UINT64_MAX / num_result_slots / 2u)
     return fail(GPJ_ERR_OUT_OF_RANGE, "result array too large");
+  const uint64_t had = ctx->compact_scratch_bytes;
   rc = ensure(ctx->compact_scratch, ctx->compact_scratch_bytes,
               gpjb::compact_scratch_bytes(num_lines, num_result_slots));
   if (rc != GPJ_OK) return rc;
+  if (ctx->compact_scratch_bytes != had)
+    GPJ_CUDA(cudaMemsetAsync(ctx->compact_scratch, 0, gpjb::kCompactHeaderBytes,
+                             static_cast<cudaStream_t>(stream_)),
+             "cudaMemsetAsync");
   GPJ_CUDA(gpjb::compact_launch(d_results, num_lines, num_result_slots, d_input, size_bytes,
                                 base_offset, d_matches, match_capacity, d_arena,
                                 arena_capacity,

@@ -9,10 +9,12 @@
 
 namespace gpjb {
 
-// Bytes of scratch compact_launch needs (per-block counts), 256-byte aligned.
+// Scratch of compact_launch: a header whose bytes are zero before the first
+// call with it (every call leaves them zero again), then per-block counts.
+constexpr uint64_t kCompactHeaderBytes = 256;
 uint64_t compact_scratch_bytes(uint64_t lines, uint32_t slots);
 
-// Clears d_counts, then: d_counts[0] = matches, [1] = arena bytes, [2] =
+// Writes d_counts[0] = matches, [1] = arena bytes, [2] =
 // invalid ranges.  Matches and bytes beyond the capacities are counted but
 // not written.  d_arena or d_input may be null (no bytes gathered).
 cudaError_t compact_launch(const int32_t *d_results, uint64_t lines, uint32_t slots,
