@@ -112,13 +112,15 @@ int bind_launch(gpj_batch *b) {
   L.NL = b->d_NL;
   L.nl_cap = b->d_NL ? b->nl_slots : 0;
   gpjb::index_bind_scratch(L, b->d_scratch);
+  L.zero[0] = reinterpret_cast<unsigned long long *>(b->d_totals + gpjb::kTotRecordCounter);
   b->tma = (b->flags & GPJ_INDEX_NO_TMA) == 0 &&
            gpjb::index_make_tensor_map(&b->map, b->d_input, b->input_bytes, b->index_threads);
   return GPJ_OK;
 }
 
-gpjb::BatchQueryLaunch query_launch_of(const gpj_batch *b) {
+gpjb::BatchQueryLaunch query_launch_of(const gpj_batch *b, bool after_index) {
   gpjb::BatchQueryLaunch q;
+  q.counter_cleared = after_index;  // with the indexer's scratch (bind_launch)
   q.in = b->d_input;
   q.S = b->d_S;
   q.LB = b->d_LB;
@@ -146,8 +148,8 @@ cudaError_t enqueue(gpj_batch *b, cudaStream_t stream, bool with_query) {
   e = gpjb::index_finalize_files(b->L, b->d_query_of_file, b->d_slots, b->d_info, b->d_totals,
                                  stream);
   if (e != cudaSuccess || !with_query) return e;
-  return gpjb::batch_query_launch(query_launch_of(b), b->blob, b->query_grid, b->query_block,
-                                  stream);
+  return gpjb::batch_query_launch(query_launch_of(b, true), b->blob, b->query_grid,
+                                  b->query_block, stream);
 }
 
 void release(gpj_batch *b) {
@@ -436,8 +438,8 @@ int gpj_batch_run_stages(gpj_batch *b, uint32_t stages, void *stream_) {
                                      b->d_totals, stream),
           "batch finalize launch");
   if (stages & GPJ_BATCH_STAGE_QUERY)
-    BCUDA(gpjb::batch_query_launch(query_launch_of(b), b->blob, b->query_grid, b->query_block,
-                                   stream),
+    BCUDA(gpjb::batch_query_launch(query_launch_of(b, false), b->blob, b->query_grid,
+                                   b->query_block, stream),
           "batch query launch");
   return GPJ_OK;
 }
@@ -548,8 +550,8 @@ int run_in_pieces(gpj_batch *b, const uint8_t *h_input, cudaStream_t stream) {
   BCUDA(gpjb::index_finalize_files(b->L, b->d_query_of_file, b->d_slots, b->d_info,
                                    b->d_totals, stream),
         "finalize launch");
-  BCUDA(gpjb::batch_query_launch(query_launch_of(b), b->blob, b->query_grid, b->query_block,
-                                 stream),
+  BCUDA(gpjb::batch_query_launch(query_launch_of(b, true), b->blob, b->query_grid,
+                                 b->query_block, stream),
         "batch query launch");
   return GPJ_OK;
 }

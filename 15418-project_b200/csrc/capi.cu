@@ -97,10 +97,21 @@ uint64_t round256(uint64_t x) { return (x + 255u) & ~uint64_t(255); }
 // is repeated with the exact size.
 uint64_t nl_capacity_guess(uint64_t n) { return n / 32u + 1024u; }
 
+// Sends the kernel's summary and error bits of a non-empty build straight to
+// the caller's four words (the error word is zeroed with the scratch).
+void bind_summary(gpjb::IndexLaunch &L, uint64_t *d_summary) {
+  L.summary = reinterpret_cast<unsigned long long *>(d_summary);
+  L.error = reinterpret_cast<unsigned int *>(d_summary + 3);
+  L.zero[0] = L.summary + 3;
+}
+
 // Enqueues the fused indexer.  `in` may be unaligned: it is then copied into
-// the context's staging buffer first (TMA needs 16-byte aligned rows).
+// the context's staging buffer first (TMA needs 16-byte aligned rows).  The
+// summary goes to d_summary where that is given and the input not empty, else
+// to the context's scratch.
 int enqueue_index(gpj_ctx *ctx, const uint8_t *in, uint64_t n, int levels,
-                  uint32_t flags, const gpj_index &out, cudaStream_t stream) {
+                  uint32_t flags, const gpj_index &out, uint64_t *d_summary,
+                  cudaStream_t stream) {
   gpjb::IndexLaunch L;
   L.single.n = n;
   L.single.levels = levels;
@@ -127,6 +138,7 @@ int enqueue_index(gpj_ctx *ctx, const uint8_t *in, uint64_t n, int levels,
   int rc = ensure(ctx->scratch, ctx->scratch_bytes, gpjb::index_scratch_bytes(n));
   if (rc != GPJ_OK) return rc;
   gpjb::index_bind_scratch(L, ctx->scratch);
+  if (n > 0 && d_summary != nullptr) bind_summary(L, d_summary);
 
   CUtensorMap map;
   bool tma = false;
@@ -243,7 +255,7 @@ int enqueue_index_from_host(gpj_ctx *ctx, const uint8_t *h_in, uint8_t *d_in, ui
   if (n <= piece) {
     const int rc = stage_copy(ctx, d_in, h_in, n, stream, pinned);
     if (rc != GPJ_OK) return rc;
-    return enqueue_index(ctx, d_in, n, levels, 0u, out, stream);
+    return enqueue_index(ctx, d_in, n, levels, 0u, out, nullptr, stream);
   }
   if (ctx->copy_stream == nullptr)
     GPJ_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking),
@@ -286,32 +298,24 @@ int enqueue_index_from_host(gpj_ctx *ctx, const uint8_t *h_in, uint8_t *d_in, ui
   return GPJ_OK;
 }
 
-// summary words in the context scratch: [lines, in_string, depth, pad] then
-// the error word
+// summary words in the context scratch: [lines, in_string, depth, pad], then
+// the ticket counter and the error word
 const unsigned long long *summary_ptr(gpj_ctx *ctx, uint64_t n) {
   gpjb::IndexLaunch L;
   L.num_tiles = uint32_t(gpjb::index_num_tiles(n));
   gpjb::index_bind_scratch(L, ctx->scratch);
   return L.summary;
 }
-const unsigned int *error_ptr(gpj_ctx *ctx, uint64_t n) {
-  gpjb::IndexLaunch L;
-  L.num_tiles = uint32_t(gpjb::index_num_tiles(n));
-  gpjb::index_bind_scratch(L, ctx->scratch);
-  return L.error;
-}
-
 // Copies the summary and error word to pinned memory and waits.
 int read_summary(gpj_ctx *ctx, uint64_t n, cudaStream_t stream, uint64_t *lines,
                  int *in_string, int *depth) {
-  GPJ_CUDA(cudaMemcpyAsync(ctx->pinned, summary_ptr(ctx, n), 32, cudaMemcpyDeviceToHost,
+  // the four summary words, the ticket counter and the error word follow one
+  // another
+  GPJ_CUDA(cudaMemcpyAsync(ctx->pinned, summary_ptr(ctx, n), 40, cudaMemcpyDeviceToHost,
                            stream),
            "read index summary");
-  GPJ_CUDA(cudaMemcpyAsync(ctx->pinned + 4, error_ptr(ctx, n), 4, cudaMemcpyDeviceToHost,
-                           stream),
-           "read index error word");
   GPJ_CUDA(cudaStreamSynchronize(stream), "cudaStreamSynchronize");
-  const unsigned int err = reinterpret_cast<const unsigned int *>(ctx->pinned + 4)[0];
+  const unsigned int err = reinterpret_cast<const unsigned int *>(ctx->pinned + 4)[1];
   if (n > 0 && err != 0)
     return fail(GPJ_ERR_TIMEOUT, "index kernel: a bounded wait gave up (error bits " +
                                      std::to_string(err) + ")");
@@ -579,7 +583,7 @@ int gpj_index_build(gpj_ctx *ctx, const uint8_t *d_input, uint64_t size_bytes,
     if (rc != GPJ_OK) return rc;
     out->d_input = d_input;
     out->size_bytes = size_bytes;
-    rc = enqueue_index(ctx, d_input, size_bytes, num_levels, flags, *out, stream);
+    rc = enqueue_index(ctx, d_input, size_bytes, num_levels, flags, *out, nullptr, stream);
     uint64_t lines = 0;
     int in_string = 0, depth = -1;
     if (rc == GPJ_OK) rc = read_summary(ctx, size_bytes, stream, &lines, &in_string, &depth);
@@ -615,17 +619,13 @@ int gpj_index_build_async(gpj_ctx *ctx, const uint8_t *d_input, uint64_t size_by
   index->size_bytes = size_bytes;
   index->num_words = W;
   index->num_levels = num_levels;
-  rc = enqueue_index(ctx, d_input, size_bytes, num_levels, flags, *index, stream);
+  rc = enqueue_index(ctx, d_input, size_bytes, num_levels, flags, *index, d_summary, stream);
   if (rc != GPJ_OK) return rc;
-  if (d_summary != nullptr) {
+  if (d_summary != nullptr && size_bytes == 0) {
     GPJ_CUDA(cudaMemcpyAsync(d_summary, summary_ptr(ctx, size_bytes), 24,
                              cudaMemcpyDeviceToDevice, stream),
              "copy summary");
     GPJ_CUDA(cudaMemsetAsync(d_summary + 3, 0, 8, stream), "cudaMemsetAsync");
-    if (size_bytes > 0)
-      GPJ_CUDA(cudaMemcpyAsync(d_summary + 3, error_ptr(ctx, size_bytes), 4,
-                               cudaMemcpyDeviceToDevice, stream),
-               "copy error word");
   }
   return GPJ_OK;
 }

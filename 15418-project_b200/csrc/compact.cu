@@ -18,6 +18,7 @@
 // byte).  What is left is bound by instructions (27 a match) and by the texts'
 // scattered sectors (35 MB read for 5 MB of text).
 #include "compact.cuh"
+#include "overlap.cuh"
 
 namespace gpjb {
 namespace {
@@ -377,18 +378,9 @@ cudaError_t compact_launch(const int32_t *d_results, uint64_t lines, uint32_t sl
       d_results, items, n, bc, uint32_t(blocks), ticket, d_counts);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  cudaLaunchConfig_t config{};
-  config.gridDim = dim3(uint32_t(blocks));
-  config.blockDim = dim3(kThreads);
-  config.stream = stream;
-  cudaLaunchAttribute overlap{};
-  overlap.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  overlap.val.programmaticStreamSerializationAllowed = 1;
-  config.attrs = &overlap;
-  config.numAttrs = 1;
-  const BlockCounts *counted = bc;
-  return cudaLaunchKernelEx(&config, write_kernel, d_results, items, slots, d_input, n,
-                            base_offset, counted, d_matches, match_cap, d_arena, arena_cap);
+  return launch_overlapped(write_kernel, uint32_t(blocks), kThreads, 0, stream, d_results, items,
+                           slots, d_input, n, base_offset, bc, d_matches, match_cap, d_arena,
+                           arena_cap);
 }
 
 }  // namespace gpjb

@@ -21,6 +21,7 @@
 #include "bits.cuh"
 #include "descriptor.cuh"
 #include "indexer.cuh"
+#include "overlap.cuh"
 
 #include <cudaTypedefs.h>
 
@@ -920,6 +921,8 @@ __global__ void __launch_bounds__(NT + 32, NT <= 128 ? 4 : 2)
   LevelScratch<NT, LMAX, kList> &ls = *reinterpret_cast<LevelScratch<NT, LMAX, kList> *>(
       smem_base + level_scratch_offset<NT>());
   const int tid = threadIdx.x;
+  // the file table's finalize kernel may be launched; it waits for this grid
+  asm volatile("griddepcontrol.launch_dependents;");
   if (tid == NT) {
     // barriers must be initialised before anyone polls them: shared memory
     // may still hold barriers of an earlier CTA on this SM
@@ -938,6 +941,10 @@ __global__ void __launch_bounds__(NT + 32, NT <= 128 ? 4 : 2)
   }
   __syncthreads();
   if (tid >= NT) {
+    // The CTA may have started while the kernel that clears the scratch ran:
+    // the tickets and descriptors are touched only from here on (the compute
+    // warps publish after the control warp has staged a tile).
+    asm volatile("griddepcontrol.wait;" ::: "memory");
     control_warp<NT, kTma, kLB>(P, sm, &tmap);
     return;
   }
@@ -965,7 +972,8 @@ __global__ void __launch_bounds__(NT + 32, NT <= 128 ? 4 : 2)
 }
 
 template <int LMAX, bool kTma, int NT, bool kList, int kLB, bool kPasses>
-cudaError_t launch_kernel(const IndexLaunch &L, const CUtensorMap &map, cudaStream_t stream) {
+cudaError_t launch_kernel(const IndexLaunch &L, const CUtensorMap &map, bool overlap,
+                          cudaStream_t stream) {
   auto kernel = index_kernel<LMAX, kTma, NT, kList, kLB, kPasses>;
   constexpr size_t smem = level_scratch_offset<NT>() + sizeof(LevelScratch<NT, LMAX, kList>) +
                           1024;  // + alignment slack
@@ -986,16 +994,19 @@ cudaError_t launch_kernel(const IndexLaunch &L, const CUtensorMap &map, cudaStre
     grid_per_device[dev] = (per_sm > 0 ? per_sm : 1) * (sms > 0 ? sms : 1);
   }
   const uint32_t grid = min(L.tile_end - L.tile_begin, uint32_t(grid_per_device[dev]));
-  kernel<<<grid, NT + 32, smem, stream>>>(map, L);
-  return cudaGetLastError();
+  if (!overlap) {
+    kernel<<<grid, NT + 32, smem, stream>>>(map, L);
+    return cudaGetLastError();
+  }
+  return launch_overlapped(kernel, grid, NT + 32, smem, stream, map, L);
 }
 
 template <int LMAX, int NT, bool kList, int kLB, bool kPasses = false>
-cudaError_t launch_tma(const IndexLaunch &L, const CUtensorMap *map, bool use_tma,
+cudaError_t launch_tma(const IndexLaunch &L, const CUtensorMap *map, bool use_tma, bool overlap,
                        cudaStream_t stream) {
-  if (use_tma) return launch_kernel<LMAX, true, NT, kList, kLB, kPasses>(L, *map, stream);
+  if (use_tma) return launch_kernel<LMAX, true, NT, kList, kLB, kPasses>(L, *map, overlap, stream);
   CUtensorMap dummy{};
-  return launch_kernel<LMAX, false, NT, kList, kLB, kPasses>(L, dummy, stream);
+  return launch_kernel<LMAX, false, NT, kList, kLB, kPasses>(L, dummy, overlap, stream);
 }
 
 // The launch variant (IndexLaunch::variant) picks the walk and the look-back
@@ -1003,30 +1014,30 @@ cudaError_t launch_tma(const IndexLaunch &L, const CUtensorMap *map, bool use_tm
 // always walk per lane with rounds of 32 descriptors.
 template <int LMAX, int NT>
 cudaError_t launch_levels(const IndexLaunch &L, const CUtensorMap *map, bool use_tma,
-                          cudaStream_t stream) {
+                          bool overlap, cudaStream_t stream) {
   if constexpr (walk_list_allowed<LMAX>()) {
     const bool lanes = (L.variant & kIndexVariantLaneWalk) != 0;
     const bool wide = (L.variant & kIndexVariantWideLookback) != 0;
-    if (lanes && wide) return launch_tma<LMAX, NT, false, 2>(L, map, use_tma, stream);
-    if (lanes) return launch_tma<LMAX, NT, false, 1>(L, map, use_tma, stream);
-    if (wide) return launch_tma<LMAX, NT, true, 2>(L, map, use_tma, stream);
-    return launch_tma<LMAX, NT, true, 1>(L, map, use_tma, stream);
+    if (lanes && wide) return launch_tma<LMAX, NT, false, 2>(L, map, use_tma, overlap, stream);
+    if (lanes) return launch_tma<LMAX, NT, false, 1>(L, map, use_tma, overlap, stream);
+    if (wide) return launch_tma<LMAX, NT, true, 2>(L, map, use_tma, overlap, stream);
+    return launch_tma<LMAX, NT, true, 1>(L, map, use_tma, overlap, stream);
   } else {
-    return launch_tma<LMAX, NT, false, 1>(L, map, use_tma, stream);
+    return launch_tma<LMAX, NT, false, 1>(L, map, use_tma, overlap, stream);
   }
 }
 
 template <int NT>
 cudaError_t launch_threads(const IndexLaunch &L, const CUtensorMap *map, bool use_tma,
-                           cudaStream_t stream) {
+                           bool overlap, cudaStream_t stream) {
   const int lv = L.num_levels;
-  if (lv <= 2) return launch_levels<2, NT>(L, map, use_tma, stream);
-  if (lv <= 4) return launch_levels<4, NT>(L, map, use_tma, stream);
-  if (lv <= kSharedLevels) return launch_levels<kSharedLevels, NT>(L, map, use_tma, stream);
+  if (lv <= 2) return launch_levels<2, NT>(L, map, use_tma, overlap, stream);
+  if (lv <= 4) return launch_levels<4, NT>(L, map, use_tma, overlap, stream);
+  if (lv <= kSharedLevels) return launch_levels<kSharedLevels, NT>(L, map, use_tma, overlap, stream);
   // 96 MiB of posts: 8 levels 81 us; in passes 12, 15 and 22 levels 103, 104
   // and 111 us (191, 193 and 197 us in an instance that held 22 levels in
   // registers and went over all of them at every bracket)
-  return launch_tma<kSharedLevels, NT, false, 1, true>(L, map, use_tma, stream);
+  return launch_tma<kSharedLevels, NT, false, 1, true>(L, map, use_tma, overlap, stream);
 }
 
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
@@ -1071,8 +1082,43 @@ bool index_make_tensor_map(CUtensorMap *map, const uint8_t *in, uint64_t n, int 
   return r == CUDA_SUCCESS;
 }
 
+namespace {
+
+constexpr int kClearThreads = 256;
+
+// Zeroes the descriptors and counters, and up to two words elsewhere.
+__global__ void __launch_bounds__(kClearThreads)
+    clear_kernel(unsigned long long *words, uint64_t count, unsigned long long *a,
+                 unsigned long long *b) {
+  asm volatile("griddepcontrol.launch_dependents;");
+  const uint64_t stride = uint64_t(gridDim.x) * kClearThreads;
+  for (uint64_t i = uint64_t(blockIdx.x) * kClearThreads + threadIdx.x; i < count; i += stride)
+    words[i] = 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (a != nullptr) *a = 0;
+    if (b != nullptr) *b = 0;
+  }
+}
+
+cudaError_t launch_range(const IndexLaunch &L, const CUtensorMap *map, bool use_tma, bool overlap,
+                         cudaStream_t stream, uint32_t t0, uint32_t t1, int threads) {
+  if (t1 > L.num_tiles) t1 = L.num_tiles;
+  if (t0 >= t1) return cudaSuccess;
+  IndexLaunch R = L;
+  R.tile_begin = t0;
+  R.tile_end = t1;
+  if (threads == 128) return launch_threads<128>(R, map, use_tma, overlap, stream);
+  return launch_threads<256>(R, map, use_tma, overlap, stream);
+}
+
+}  // namespace
+
 cudaError_t index_clear_scratch(const IndexLaunch &L, cudaStream_t stream) {
-  return cudaMemsetAsync(L.tile_state, 0, uint64_t(L.num_tiles) * 8u + 64u, stream);
+  const uint64_t words = uint64_t(L.num_tiles) + 8u;
+  const uint64_t blocks = (words + kClearThreads - 1) / kClearThreads;
+  clear_kernel<<<uint32_t(blocks < 148u ? blocks : 148u), kClearThreads, 0, stream>>>(
+      L.tile_state, words, L.zero[0], L.zero[1]);
+  return cudaGetLastError();
 }
 
 cudaError_t index_clear_counter(const IndexLaunch &L, cudaStream_t stream) {
@@ -1081,21 +1127,14 @@ cudaError_t index_clear_counter(const IndexLaunch &L, cudaStream_t stream) {
 
 cudaError_t index_launch_range(const IndexLaunch &L, const CUtensorMap *map, bool use_tma,
                                cudaStream_t stream, uint32_t t0, uint32_t t1, int threads) {
-  if (t1 > L.num_tiles) t1 = L.num_tiles;
-  if (t0 >= t1) return cudaSuccess;
-  IndexLaunch R = L;
-  R.tile_begin = t0;
-  R.tile_end = t1;
-  if (threads == 128) return launch_threads<128>(R, map, use_tma, stream);
-  return launch_threads<256>(R, map, use_tma, stream);
+  return launch_range(L, map, use_tma, false, stream, t0, t1, threads);
 }
 
 cudaError_t index_launch(const IndexLaunch &L, const CUtensorMap *map, bool use_tma,
                          cudaStream_t stream, int threads) {
-  if (L.num_tiles == 0) return cudaSuccess;
-  cudaError_t e = index_clear_scratch(L, stream);
-  if (e != cudaSuccess) return e;
-  return index_launch_range(L, map, use_tma, stream, 0u, L.num_tiles, threads);
+  const cudaError_t e = index_clear_scratch(L, stream);
+  if (e != cudaSuccess || L.num_tiles == 0) return e;
+  return launch_range(L, map, use_tma, true, stream, 0u, L.num_tiles, threads);
 }
 }  // namespace gpjb
 
@@ -1110,6 +1149,8 @@ __global__ void __launch_bounds__(kFinalizeThreads)
   __shared__ unsigned long long s_warp_rec[32], s_warp_out[32];
   __shared__ unsigned long long s_carry_rec, s_carry_out;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  asm volatile("griddepcontrol.launch_dependents;");  // the batch query
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // the index
   if (tid == 0) {
     s_carry_rec = 0;
     s_carry_out = 0;
@@ -1193,9 +1234,8 @@ __global__ void __launch_bounds__(kFinalizeThreads)
 cudaError_t index_finalize_files(const IndexLaunch &L, const uint32_t *query_of_file,
                                  const uint32_t *slots_of_query, uint64_t *file_info,
                                  uint64_t *totals, cudaStream_t stream) {
-  finalize_files_kernel<<<1, kFinalizeThreads, 0, stream>>>(L, query_of_file, slots_of_query,
-                                                             file_info, totals);
-  return cudaGetLastError();
+  return launch_overlapped(finalize_files_kernel, 1u, kFinalizeThreads, 0, stream, L,
+                           query_of_file, slots_of_query, file_info, totals);
 }
 
 }  // namespace gpjb

@@ -52,6 +52,8 @@ struct IndexLaunch {
   unsigned int *tile_counter = nullptr;
   unsigned int *error = nullptr;
   unsigned long long *summary = nullptr;  // [0] lines [1] in-string [2] depth
+  // words outside the scratch that index_clear_scratch zeroes too (optional)
+  unsigned long long *zero[2] = {nullptr, nullptr};
   uint32_t num_tiles = 0;
   // tiles this launch claims: [tile_begin, tile_end); set by the launchers
   uint32_t tile_begin = 0, tile_end = 0;
@@ -99,7 +101,9 @@ bool index_make_tensor_map(CUtensorMap *map, const uint8_t *in, uint64_t n,
 
 // Zeroes the scratch and launches the indexer on `stream` with `threads`
 // (128 or 256) threads per CTA: tiles of threads * 128 bytes, so num_tiles
-// and the files' first tiles must be counted with that tile size.
+// and the files' first tiles must be counted with that tile size.  The
+// indexer's launch overlaps the clearing kernel; every access to the scratch
+// waits for it.
 cudaError_t index_launch(const IndexLaunch &L, const CUtensorMap *map,
                          bool use_tma, cudaStream_t stream,
                          int threads = kIndexThreads);
@@ -149,7 +153,8 @@ enum TotalField : int {
 // After index_launch on a file table: derives every file's line count,
 // newline-index slot, record and result offsets (exclusive scans over the
 // files) from the tiles' inclusive look-back descriptors, writes the leading
-// 0 of each empty file's newline index, and the totals.  One CTA.
+// 0 of each empty file's newline index, and the totals.  One CTA, launched
+// while a kernel before it on the stream still runs; it waits for that.
 cudaError_t index_finalize_files(const IndexLaunch &L, const uint32_t *query_of_file,
                                  const uint32_t *slots_of_query, uint64_t *file_info,
                                  uint64_t *totals, cudaStream_t stream);

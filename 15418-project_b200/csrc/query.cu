@@ -7,6 +7,7 @@
 // streams do not race.  Positions are 32-bit for partitions below 2 GiB (every
 // value equals the reference's int arithmetic) and 64-bit beyond.
 #include "query.cuh"
+#include "overlap.cuh"
 
 #include <algorithm>
 
@@ -1057,6 +1058,8 @@ __global__ void __launch_bounds__(256, 4)
     if (threadIdx.x == 0) s_ir_off[k] = off;
     off += (len + kIrPad + 3) & ~3;
   }
+  // launched while the finalize kernel runs; its rows and totals from here on
+  asm volatile("griddepcontrol.wait;" ::: "memory");
   __syncthreads();
   __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed];
   const Group<G> g;
@@ -1265,8 +1268,8 @@ int lanes_per_record(uint64_t records, bool descends) {
 template <int G>
 void batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, bool ext, int nlev, int grid,
                        int block, size_t smem, cudaStream_t stream) {
-  if (ext) batch_query_kernel<true, G><<<grid, block, smem, stream>>>(q, ir, nlev);
-  else batch_query_kernel<false, G><<<grid, block, smem, stream>>>(q, ir, nlev);
+  launch_overlapped(ext ? batch_query_kernel<true, G> : batch_query_kernel<false, G>,
+                    uint32_t(grid), uint32_t(block), smem, stream, q, ir, nlev);
 }
 
 template <typename Pos, typename OutT, int G>
@@ -1314,7 +1317,7 @@ cudaError_t batch_query_launch(const BatchQueryLaunch &q, const IrBlob &ir, int 
     grid = int(std::min<uint64_t>(uint64_t(grid), blocks));
   }
   const size_t smem = size_t(nlev + marks) * size_t(block) * sizeof(int32_t);
-  if (q.record_counter != nullptr) {
+  if (q.record_counter != nullptr && !q.counter_cleared) {
     const cudaError_t e = cudaMemsetAsync(q.record_counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
   }

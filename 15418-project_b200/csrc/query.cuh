@@ -76,8 +76,10 @@ struct BatchQueryLaunch {
   unsigned int *status = nullptr;  // kQueryStatusOverflow is OR-ed here (optional)
   unsigned int *file_status = nullptr;  // or into one word per file (optional, first)
   // records are handed to warps from this counter, which the launch zeroes
-  // first (optional; without it each warp strides)
+  // first unless the kernels before it did (optional; without it each warp
+  // strides)
   unsigned long long *record_counter = nullptr;
+  bool counter_cleared = false;
   // about the number of records (0: unknown, many): chooses the lanes per
   // record and bounds the grid; the results do not depend on it
   uint64_t expected_records = 0;
