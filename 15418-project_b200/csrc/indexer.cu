@@ -1149,8 +1149,7 @@ __global__ void __launch_bounds__(kFinalizeThreads)
   __shared__ unsigned long long s_warp_rec[32], s_warp_out[32];
   __shared__ unsigned long long s_carry_rec, s_carry_out;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  asm volatile("griddepcontrol.launch_dependents;");  // the batch query
-  asm volatile("griddepcontrol.wait;" ::: "memory");  // the index
+  asm volatile("griddepcontrol.wait;" ::: "memory");  // for the index
   if (tid == 0) {
     s_carry_rec = 0;
     s_carry_out = 0;
