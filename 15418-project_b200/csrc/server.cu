@@ -29,6 +29,7 @@
 // after the event that follows its last use has completed.
 #include "indexer.cuh"
 #include "query.cuh"
+#include "copies.cuh"
 
 #include "gpjson_b200.h"
 
@@ -1009,9 +1010,9 @@ struct gpj_server {
       ir_off += int(gr->irs[gq].size());
     }
     Slot &s0 = slots[in_batch[0]->slot];
-    cudaError_t e = cudaMemcpyAsync(d_files, h_files, files_bytes + V * 64u + 32u,
-                                    cudaMemcpyHostToDevice, s0.stream);
-    if (e == cudaSuccess) e = cudaMemsetAsync(d_stat, 0, V * 4u, s0.stream);
+    const gpjb::CopyItem tables[] = {{h_files, d_files, files_bytes + V * 64u + 32u},
+                                     {nullptr, d_stat, V * 4u}};
+    cudaError_t e = gpjb::copy_many(tables, 2, s0.stream);
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device);
     ql.expected_records = records;
@@ -1019,21 +1020,29 @@ struct gpj_server {
       e = gpjb::batch_query_launch(ql, blob, std::max(sms, 1) * 8, 128, s0.stream);
     b->refs = int(in_batch.size());
     qbatches.emplace(b, std::move(owned));
+    // every request's status words and, where they are small, its results go
+    // to the host in one launch
+    std::vector<gpjb::CopyItem> out;
     uint64_t v = 0;
+    for (Request *r : in_batch) {
+      const uint64_t bytes = r->res->lines * r->slots_total * 8u;
+      const uint32_t nq = uint32_t(r->queries.size());
+      out.push_back({d_stat + v, slots[r->slot].pinned + 4, nq * 4u});
+      v += nq;
+      if (bytes > 0 && bytes <= gpjb::kCopyManyMaxResult)
+        out.push_back({dptr(r->work_off + r->scratch_bytes), h_arena + r->host_off / 4u, bytes});
+    }
+    if (e == cudaSuccess) e = gpjb::copy_many(out.data(), int(out.size()), s0.stream);
     for (Request *r : in_batch) {
       Slot &s = slots[r->slot];
       const uint64_t ints = r->res->lines * r->slots_total * 2u;
       const uint32_t nq = uint32_t(r->queries.size());
       r->qbatch = b;
       r->status_words = nq;
-      if (e == cudaSuccess && ints > 0)
+      if (e == cudaSuccess && ints * 4u > gpjb::kCopyManyMaxResult)
         e = cudaMemcpyAsync(h_arena + r->host_off / 4u, dptr(r->work_off + r->scratch_bytes),
                             ints * 4u, cudaMemcpyDeviceToHost, s0.stream);
-      if (e == cudaSuccess)
-        e = cudaMemcpyAsync(reinterpret_cast<unsigned int *>(s.pinned + 4), d_stat + v, nq * 4u,
-                            cudaMemcpyDeviceToHost, s0.stream);
       if (e == cudaSuccess) e = cudaEventRecord(s.event, s0.stream);
-      v += nq;
       r->resp.num_lines = r->res->lines;
       r->resp.result_ints = ints;
       r->state = St::Querying;
@@ -1202,13 +1211,20 @@ struct gpj_server {
     gpjb::index_bind_scratch(L, dptr(g->meta_off + files_bytes));
     Slot &s = slots[members[0]->slot];
     cudaError_t e = cudaSuccess;
-    for (Request *r : members)
-      if (e == cudaSuccess && r->res->size > 0)
-        e = cudaMemcpyAsync(r->res->d_input, r->h_input, r->res->size, cudaMemcpyHostToDevice,
-                            s.stream);
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(d_files, h_files, uint64_t(G) * sizeof(gpjb::IndexFile),
-                          cudaMemcpyHostToDevice, s.stream);
+    // the file table and the small pinned inputs in one launch
+    std::vector<gpjb::CopyItem> in;
+    in.push_back({h_files, d_files, uint64_t(G) * sizeof(gpjb::IndexFile)});
+    for (Request *r : members) {
+      const uint64_t size = r->res->size;
+      if (size == 0) continue;
+      if (size <= gpjb::kCopyManyMaxInput &&
+          (reinterpret_cast<uintptr_t>(r->h_input) & 15u) == 0 &&
+          gpjb::host_range_mapped(r->h_input, size))
+        in.push_back({r->h_input, r->res->d_input, size});
+      else if (e == cudaSuccess)
+        e = cudaMemcpyAsync(r->res->d_input, r->h_input, size, cudaMemcpyHostToDevice, s.stream);
+    }
+    if (e == cudaSuccess) e = gpjb::copy_many(in.data(), int(in.size()), s.stream);
     if (e == cudaSuccess && tiles > 0)
       e = gpjb::index_launch(L, arena_tma ? &arena_map : nullptr, arena_tma, s.stream);
     if (e == cudaSuccess && tiles == 0)
