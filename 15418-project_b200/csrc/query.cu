@@ -488,7 +488,16 @@ __device__ __forceinline__ bool find_key_lane(const Rec<Pos> &c, const Query &q,
 
 // Structural characters a group looks at in one round, at most (a word has at
 // most 64).
-constexpr int kListed = 64;
+template <int G>
+constexpr int kListed = G == 32 ? 256 : 64;
+
+// One lane.  Writes the positions of a word's set bits, plus `first`.
+__device__ __forceinline__ void list_bits(uint16_t *list, uint64_t word, int first) {
+  for (uint32_t m = uint32_t(word); m != 0; m &= m - 1)
+    *list++ = uint16_t(first + __ffs(int(m)) - 1);
+  for (uint32_t m = uint32_t(word >> 32); m != 0; m &= m - 1)
+    *list++ = uint16_t(first + 31 + __ffs(int(m)));
+}
 
 // The key search of MOVE_TO_KEY (query.cu:254-302) for every active record of
 // the warp.  The structural characters after line_index, up to level_end, come
@@ -553,17 +562,11 @@ __device__ bool find_key(const Rec<Pos> &c, const Query &q, const Group<G> &g, b
     int total;
     int at_slot = g.sum_before(mine, total);
     int words = G;
-    if (__any_sync(kAll, total > kListed)) {  // more than a round's: fewer words
-      words = __popc(g.ballot(g.lane == 0 || at_slot + mine <= kListed));
+    if (__any_sync(kAll, total > kListed<G>)) {  // more than a round's: fewer words
+      words = __popc(g.ballot(g.lane == 0 || at_slot + mine <= kListed<G>));
       total = g.shfl(at_slot + mine, words - 1);
     }
-    if (g.lane < words) {
-      const int first = g.lane * 64;
-      for (uint32_t m = uint32_t(cand); m != 0; m &= m - 1)
-        list[at_slot++] = uint16_t(first + __ffs(int(m)) - 1);
-      for (uint32_t m = uint32_t(cand >> 32); m != 0; m &= m - 1)
-        list[at_slot++] = uint16_t(first + 31 + __ffs(int(m)));
-    }
+    if (g.lane < words) list_bits(list + at_slot, cand, g.lane * 64);
     __syncwarp();
     const Pos base = w0 * 64;
     const uint8_t *text = c.in + base;
@@ -617,6 +620,90 @@ __device__ bool find_key(const Rec<Pos> &c, const Query &q, const Group<G> &g, b
   return found;
 }
 
+// "..name" by a whole warp: every member named key inside (line_index,
+// level_end), at any level from `level` up, in document order (by the position
+// of its ':').  The lanes list the structural characters of all those levels
+// in their words, test one each for the key, and collect the few that match;
+// those are then resolved one per lane.  (Each lane testing the characters of
+// its own word left two thirds of the lanes idle: 41 K records 231 us, so 200.)
+// Returns `stored` plus the matches.
+template <typename Pos, typename OutT>
+__device__ int descend(const Rec<Pos> &c, const Query &q, const Group<32> &g, Pos line_start,
+                       Pos line_index, Pos level_end, int level, const Key &key, int stored,
+                       OutT *out, uint16_t *list, Pos *matches) {
+  int waiting = 0;  // collected matches
+  auto resolve = [&] {
+    __syncwarp();
+    if (g.lane < waiting) {
+      const Pos p = matches[g.lane];
+      const int slot = stored + g.lane;
+      if (slot >= q.num_results) {
+        raise_status(c, kQueryStatusOverflow);
+      } else {
+        int l = level;
+        while (l < c.levels && (level_words(c, l) == nullptr ||
+                                ((level_words(c, l)[p >> 6] >> (p & 63)) & 1ull) == 0ull))
+          ++l;
+        const Pos vend = next_struct_lane(c, level_end, Pos(p + 1), level_words(c, l));
+        Pos vs = p + 1;
+        while (at(c, vs) == ' ' && vs < vend) ++vs;
+        Pos ve = vend;
+        while (ve > vs && at(c, ve - 1) == ' ') --ve;
+        out[2 * slot] = OutT(vs);
+        out[2 * slot + 1] = OutT(ve);
+      }
+    }
+    stored += waiting;
+    waiting = 0;
+    __syncwarp();
+  };
+  const int lowest = level > 0 ? level : 0;
+  const Pos last = min(Pos((level_end - 1) >> 6), Pos(c.W - 1));
+  for (Pos w0 = line_index >> 6; w0 <= last;) {
+    const Pos w = w0 + g.lane;
+    uint64_t cand = 0, s_word = 0;
+    if (w >= 0 && w <= last) {
+      const uint64_t *row = c.LB + uint64_t(c.W) * uint64_t(lowest) + w;
+#pragma unroll 4
+      for (int l = lowest; l < c.levels; ++l, row += c.W) cand |= *row;
+      s_word = c.S[w];
+      if (w == (line_index >> 6)) cand &= ~0ull << (line_index & 63);
+      if (w == (level_end >> 6)) cand &= (1ull << (level_end & 63)) - 1ull;
+    }
+    const int mine = __popcll(cand);
+    int total;
+    int at_slot = g.sum_before(mine, total);
+    int words = 32;
+    if (total > kListed<32>) {
+      words = __popc(g.ballot(g.lane == 0 || at_slot + mine <= kListed<32>));
+      total = g.shfl(at_slot + mine, words - 1);
+    }
+    if (g.lane < words) list_bits(list + at_slot, cand, g.lane * 64);
+    __syncwarp();
+    const Pos base = w0 * 64;
+    const uint8_t *text = c.in + base;
+    for (int e0 = 0; e0 < total; e0 += 32) {
+      const bool has = e0 + g.lane < total;
+      const int o = has ? int(list[e0 + g.lane]) : 0;
+      const uint8_t b = has ? text[o] : uint8_t(0);
+      uint64_t s = __shfl_sync(kAll, (unsigned long long)s_word, (o - 1) >> 6);
+      if (has && o == 0) s = string_word_before(c, base);
+      const bool match =
+          b == ':' && key_at_colon(c, q, line_start, Pos(base + o), s, key);
+      __syncwarp();
+      const unsigned hits = g.ballot(match);
+      if (hits == 0) continue;
+      if (waiting + __popc(hits) > 32) resolve();
+      if (match) matches[waiting + __popc(hits & ((1u << g.lane) - 1u))] = base + o;
+      waiting += __popc(hits);
+    }
+    w0 += words;
+    __syncwarp();
+  }
+  resolve();
+  return stored;
+}
+
 // One lane.  Commas among the structural characters after line_index, up to
 // the first that is none or `limit` of them.
 template <typename Pos>
@@ -638,7 +725,7 @@ __device__ int count_commas(const Rec<Pos> &c, Pos max_steps, Pos level_end, con
 template <typename Pos, typename OutT, bool kExt, int G>
 __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g, bool alive,
                             Pos line_start, Pos line_end, OutT *out, Pos *ends, Pos *marks,
-                            int stride, uint16_t *list) {
+                            int stride, uint16_t *list, Pos *matches) {
   // every lane keeps its own copy of its record's state, so no lane reads
   // what another wrote, except the result slots
   if (alive)
@@ -890,71 +977,19 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       break;
     }
     case OP_DESCEND_KEY: {
-      if constexpr (!kExt) return;
-      const int key_len = read_varint(q, qp, operand);
-      const int key_pos = qp;
-      qp += key_len;
-      if (key_len < 0 || !LEVEL_OK(level)) return;
-      // every member named key inside the current value, at any level the
-      // index holds, in document order (by the position of its ':'): each
-      // lane looks at one word of all levels, and a scan over the lanes' match
-      // counts gives every match its slot
-      const Key key(q, key_pos, key_len);
-      const Pos hi = ends[level * stride];
-      const Pos last = min(Pos((hi - 1) >> 6), Pos(c.W - 1));
-      Pos w0 = line_index >> 6;
-      for (bool need = alive && w0 <= last; __any_sync(kAll, need);) {
-        const Pos w = w0 + g.lane;
-        const bool inside = need && w >= 0 && w <= last;
-        const Pos base = inside ? w * 64 : Pos(0);
-        uint64_t cand = 0, matches = 0;
-        if (inside) {
-          for (int l = q.base + level; l < c.levels; ++l) {
-            const uint64_t *lw = level_words(c, l);
-            if (lw != nullptr) cand |= lw[w];
-          }
-          if (line_index > base) cand &= ~0ull << (line_index - base);
-          if (hi - base < 64) cand &= (1ull << (hi - base)) - 1ull;
-        }
-        const uint64_t s_word = cand != 0 ? c.S[w] : 0ull;
-        for (; cand != 0; cand &= cand - 1) {
-          const int bit = __ffsll(static_cast<long long>(cand)) - 1;
-          if (c.in[base + bit] == ':' &&
-              key_at_colon(c, q, line_start, Pos(base + bit),
-                           bit > 0 ? s_word : string_word_before(c, Pos(base + bit)), key))
-            matches |= 1ull << bit;
-        }
-        __syncwarp();
-        int total = 0;
-        int slot = stored + g.sum_before(__popcll(matches), total);
-        __syncwarp();  // the slots were cleared by other lanes
-        for (; matches != 0; matches &= matches - 1, ++slot) {
-          const int bit = __ffsll(static_cast<long long>(matches)) - 1;
-          const Pos p = base + bit;
-          if (slot >= q.num_results) {
-            raise_status(c, kQueryStatusOverflow);
-            continue;
-          }
-          int l = q.base + level;
-          while (l < c.levels && (level_words(c, l) == nullptr ||
-                                  ((level_words(c, l)[w] >> bit) & 1ull) == 0ull))
-            ++l;
-          const Pos vend = next_struct_lane(c, hi, Pos(p + 1), level_words(c, l));
-          Pos vs = p + 1;
-          while (at(c, vs) == ' ' && vs < vend) ++vs;
-          Pos ve = vend;
-          while (ve > vs && at(c, ve - 1) == ' ') --ve;
-          out[2 * slot] = OutT(vs);
-          out[2 * slot + 1] = OutT(ve);
-        }
-        __syncwarp();
-        if (need) {
-          stored += total;
-          w0 += G;
-          need = w0 <= last;
-        }
+      // (lanes_per_record gives IR with this opcode a whole warp)
+      if constexpr (!kExt || G != 32) {
+        return;
+      } else {
+        const int key_len = read_varint(q, qp, operand);
+        const int key_pos = qp;
+        qp += key_len;
+        if (key_len < 0 || !LEVEL_OK(level)) return;
+        if (alive)
+          stored = descend(c, q, g, line_start, line_index, ends[level * stride], q.base + level,
+                           Key(q, key_pos, key_len), stored, out, list, matches);
+        break;
       }
-      break;
     }
     case OP_EXPECT_AT_MOST: {
       if constexpr (!kExt) return;
@@ -1006,7 +1041,8 @@ __global__ void __launch_bounds__(256, sizeof(Pos) == 8 ? 3 : (G == 1 ? 5 : 4))
   for (int i = threadIdx.x; i < q.ir_len + kIrPad; i += blockDim.x)
     s_ir[i] = i < q.ir_len ? ir.bytes[i] : uint8_t(0);
   __syncthreads();
-  __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed];
+  __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed<G>];
+  __shared__ Pos s_match[kExt && G == 32 ? 8 : 1][32];
   const Group<G> g;
   const Rec<Pos> c{q.in, Pos(q.n), q.S, q.LB, Pos(q.W), q.num_levels, q.status};
   const Query query{s_ir, q.ir_len, q.num_results, q.base_level, nlev};
@@ -1021,7 +1057,8 @@ __global__ void __launch_bounds__(256, sizeof(Pos) == 8 ? 3 : (G == 1 ? 5 : 4))
     const int64_t end = alive && r + 1 < q.num_lines ? q.NL[r + 1] : q.n - 1;
     run_records<Pos, OutT, kExt, G>(c, query, g, alive, Pos(start), Pos(end),
                                     out + r * int64_t(q.num_results) * 2, ends, marks,
-                                    int(blockDim.x), s_list[G > 1 ? threadIdx.x / G : 0]);
+                                    int(blockDim.x), s_list[G > 1 ? threadIdx.x / G : 0],
+            s_match[kExt && G == 32 ? threadIdx.x / 32 : 0]);
     __syncwarp();
   }
 }
@@ -1058,7 +1095,8 @@ __global__ void __launch_bounds__(256, 4)
     off += (len + kIrPad + 3) & ~3;
   }
   __syncthreads();
-  __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed];
+  __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed<G>];
+  __shared__ int32_t s_match[kExt && G == 32 ? 8 : 1][32];
   const Group<G> g;
   int32_t *ends = reinterpret_cast<int32_t *>(s_state) + threadIdx.x;
   int32_t *marks = ends + nlev * blockDim.x;
@@ -1108,7 +1146,8 @@ __global__ void __launch_bounds__(256, 4)
         run_records<int32_t, int32_t, kExt, G>(
             c, query, g, mine, start, end,
             q.out + row[kFiOutOff] + i * uint64_t(grp.num_results) * 2u, ends, marks,
-            int(blockDim.x), s_list[G > 1 ? threadIdx.x / G : 0]);
+            int(blockDim.x), s_list[G > 1 ? threadIdx.x / G : 0],
+            s_match[kExt && G == 32 ? threadIdx.x / 32 : 0]);
         __syncwarp();
         pending = pending && !mine;
       }
@@ -1219,10 +1258,42 @@ bool query_ir_uses_extensions(const uint8_t *ir, int len) {
 
 namespace {
 
+// Does the interpreter come across DESCEND_KEY?  Follows the IR as the kernel
+// does (operands of up to five bytes, a fifth with the high bit reads as -1;
+// zero bytes past the end).
 bool query_ir_descends(const uint8_t *ir, int len) {
-  // "..name" is always an IR's last step: a byte of a key may only add to it
-  for (int p = 0; p < len; ++p)
-    if (ir[p] == OP_DESCEND_KEY) return true;
+  int p = 0;
+  auto byte_at = [&](int i) -> uint32_t { return i < len ? ir[i] : 0u; };
+  auto varint = [&]() -> int {
+    uint32_t v = 0, b = 0;
+    for (int shift = 0;;) {
+      b = byte_at(p++);
+      if ((b & 0x80u) == 0) return int(v | (b << shift));
+      v |= (b & 0x7Fu) << shift;
+      shift += 7;
+      if (shift > 28) return -1;
+    }
+  };
+  while (p <= len + 1) {
+    const uint32_t op = byte_at(p++);
+    switch (op) {
+    case OP_END: return false;
+    case OP_DESCEND_KEY: return true;
+    case OP_NUMBER_COMPARE: ++p; [[fallthrough]];
+    case OP_MOVE_TO_KEY:
+    case OP_EXPRESSION_STRING_EQUALS: {
+      const int n = varint();
+      if (n < 0 || n > len) return false;  // the kernel stops there too
+      p += n;
+      break;
+    }
+    case OP_MOVE_TO_INDEX:
+    case OP_MOVE_TO_INDEX_REVERSE:
+    case OP_EXPECT_AT_MOST:
+    case OP_EXPECT_FOLLOWING: varint(); break;
+    default: break;
+    }
+  }
   return false;
 }
 
@@ -1252,7 +1323,7 @@ uint64_t resident_threads() {
 // (eight-slot arrays) 14 K records 90 / 83 / 127 / 163 (110), 28 K 115 / 165 /
 // 218 / 293 (140).  "..name" reads every level's words of the whole record,
 // which only a wide group reads in whole sectors: 41 K records 897 us with one
-// lane, 293 with 8, 231 with 32.
+// lane, 293 with 8, 231 with 32 (200 with the search of descend).
 int lanes_per_record(uint64_t records, bool descends) {
   if (descends) return 32;
   if (records == 0) return 1;
