@@ -276,10 +276,19 @@ __device__ __forceinline__ Agg tile_aggregate(uint32_t par, uint32_t dd, uint32_
 // file-wide prefix; it ends by publishing the tile's look-back aggregate) and
 // then phase B of tile k-1 (string mask, leveled bitmaps, newline index:
 // everything that does).  The control warp claims the CTA's next tile the
-// moment phase A of the current one ends, stages it into the free one of two
-// shared-memory buffers with a TMA tensor load, and resolves the prefix of
-// the current tile by decoupled look-back while the compute warps run phase
-// B of the previous tile and phase A of the next.
+// moment phase A of the current one ends, stages it into the buffer that this
+// phase has read with a TMA tensor load, and resolves the prefix of the current
+// tile by decoupled look-back while the compute warps run phase B of the
+// previous tile and phase A of the next.
+//
+// What bounds it is the integer work of the compute warps (about 1,380
+// instructions per 4 KiB and warp) and how well the warps of an SM cover each
+// other's latencies and barriers.  One buffer per CTA (a tile's copy has phase
+// B of the previous tile to arrive) and 72 registers a thread (36 bytes
+// spilled) put three CTAs of 256 threads on an SM: 1 GiB of products 566 ->
+// 528 us, of posts 591 -> 554 us against two CTAs with two buffers and 96
+// registers; three CTAs of 192 threads, with smaller tiles, were slower than
+// two of 256 (600 us).
 //
 // Claiming just in time keeps the time from a tile's claim to its aggregate
 // the same for every CTA (phase B of one tile plus phase A of the next), so
@@ -288,7 +297,6 @@ __device__ __forceinline__ Agg tile_aggregate(uint32_t par, uint32_t dd, uint32_
 // increasing order per CTA, and a CTA's compute warps always work on its
 // smallest unfinished tile, so every wait ends.
 // ----------------------------------------------------------------------------
-constexpr int kStages = 2;
 constexpr uint32_t kEndTile = 0xFFFFFFFFu;
 
 struct StageMeta {  // written by the control warp with each fill
@@ -323,11 +331,11 @@ constexpr uint32_t kTileInside = 1u, kTileSAligned = 2u, kTileAllAligned = 4u,
 template <int NT>
 struct PipeSmem {
   static constexpr int NW = NT / 32;
-  uint8_t tiles[kStages][NT * 128];
-  unsigned long long full[kStages];
+  uint8_t tile[NT * 128];
+  unsigned long long full;
   unsigned long long agg[2];
   unsigned long long pref[2];
-  StageMeta stage[kStages];
+  StageMeta stage;
   TileMeta tm[2];
   uint32_t last_tp[NW], warp_par[NW], warp_dd[NW], warp_nl[NW];
   uint32_t abort;
@@ -367,22 +375,22 @@ __host__ __device__ constexpr size_t level_scratch_offset() {
   return (sizeof(PipeSmem<NT>) + 15u) & ~size_t(15);
 }
 
-// Claims the next tile and stages it into buffer s (warp-collective).
+// Claims the next tile and stages it into the buffer (warp-collective).
 template <int NT, bool kTma>
 __device__ __forceinline__ void control_fill(const IndexLaunch &P, PipeSmem<NT> &sm,
-                                             const CUtensorMap *tmap, int s, bool &ended,
+                                             const CUtensorMap *tmap, bool &ended,
                                              uint32_t &tile_out) {
   constexpr uint64_t TILE_BYTES = uint64_t(NT) * 128u;
   const int lane = threadIdx.x & 31;
   uint32_t t = 0;
   if (lane == 0) t = P.tile_begin + atomicAdd(P.tile_counter, 1u);
   t = __shfl_sync(0xFFFFFFFFu, t, 0);
-  const uint32_t full = smem_u32(&sm.full[s]);
+  const uint32_t full = smem_u32(&sm.full);
   if (t >= P.tile_end) {
     ended = true;
     tile_out = kEndTile;
     if (lane == 0) {
-      sm.stage[s].tile = kEndTile;
+      sm.stage.tile = kEndTile;
       mbar_arrive(full);
       mbar_arrive(full);
     }
@@ -439,7 +447,7 @@ __device__ __forceinline__ void control_fill(const IndexLaunch &P, PipeSmem<NT> 
       mbar_arrive_tx(full, uint32_t(TILE_BYTES));
       asm volatile(
           "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes"
-          " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(sm.tiles[s])),
+          " [%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(sm.tile)),
           "l"(tmap), "r"(0), "r"(int32_t(row0)), "r"(full)
           : "memory");
       if (pf_row != ~0ull && (pf_row + NT) * 128u <= P.full_rows * 128u)
@@ -469,12 +477,12 @@ __device__ __forceinline__ void control_fill(const IndexLaunch &P, PipeSmem<NT> 
     uint32_t smem_rows = 0;
     if (kTma && row0 < P.full_rows)
       smem_rows = uint32_t(min(uint64_t(valid / 128u), P.full_rows - row0));
-    sm.stage[s].tile = t;
-    sm.stage[s].file_idx = f;
-    sm.stage[s].F = F;
-    sm.stage[s].halo = halo;
-    sm.stage[s].valid = valid;
-    sm.stage[s].smem_rows = smem_rows;
+    sm.stage.tile = t;
+    sm.stage.file_idx = f;
+    sm.stage.F = F;
+    sm.stage.halo = halo;
+    sm.stage.valid = valid;
+    sm.stage.smem_rows = smem_rows;
     mbar_arrive(full);
   }
   tile_out = t;
@@ -485,13 +493,12 @@ __device__ void control_warp(const IndexLaunch &P, PipeSmem<NT> &sm, const CUten
   static_assert(kLB == 1 || kLB == 2, "look-back descriptors per lane");
   const int lane = threadIdx.x & 31;
   const volatile uint32_t *abort = &sm.abort;
-  uint32_t stage_tile[kStages] = {kEndTile, kEndTile};
+  uint32_t staged = kEndTile;  // the tile in the buffer, or on its way there
   bool ended = false;
-  control_fill<NT, kTma>(P, sm, tmap, 0, ended, stage_tile[0]);
+  control_fill<NT, kTma>(P, sm, tmap, ended, staged);
   uint32_t k = 0;
   for (;; ++k) {
-    const int s = int(k & 1u);
-    const uint32_t tile = stage_tile[s];
+    const uint32_t tile = staged;
     if (tile == kEndTile) break;
     const int j = int(k & 1u);
     if (!mbar_wait(smem_u32(&sm.agg[j]), (k >> 1) & 1u, abort)) {
@@ -501,10 +508,10 @@ __device__ void control_warp(const IndexLaunch &P, PipeSmem<NT> &sm, const CUten
       }
       break;
     }
-    // phase A of tile k is done: claim and stage tile k+1 at once (the
-    // other buffer was read by phase A of tile k-1), then resolve k's prefix
-    if (!ended) control_fill<NT, kTma>(P, sm, tmap, s ^ 1, ended, stage_tile[s ^ 1]);
-    stage_tile[s] = kEndTile;
+    // phase A of tile k is done and with it the buffer: claim and stage tile
+    // k+1 at once, then resolve k's prefix
+    staged = kEndTile;
+    if (!ended) control_fill<NT, kTma>(P, sm, tmap, ended, staged);
 
     TileMeta &tm = sm.tm[j];
     const IndexFile F = tm.F;
@@ -528,15 +535,11 @@ __device__ void control_warp(const IndexLaunch &P, PipeSmem<NT> &sm, const CUten
     __syncwarp();
   }
   // no TMA may still be writing this CTA's shared memory when it exits: a
-  // staged tile not yet consumed is the one of iteration k (buffer k & 1) or
-  // k + 1 (the other buffer)
+  // staged tile not yet consumed is that of iteration k (no aggregate came) or
+  // k + 1 (the loop ended after staging it)
   if constexpr (kTma) {
-#pragma unroll
-    for (int s = 0; s < kStages; ++s) {
-      if (stage_tile[s] == kEndTile) continue;
-      const uint32_t kk = (uint32_t(s) == (k & 1u)) ? k : k + 1u;
-      for (uint32_t polls = 0; !mbar_try(smem_u32(&sm.full[s]), (kk >> 1) & 1u) &&
-                               polls < kSpinLimit;
+    if (staged != kEndTile) {
+      for (uint32_t polls = 0; !mbar_try(smem_u32(&sm.full), k & 1u) && polls < kSpinLimit;
            ++polls) {
       }
     }
@@ -544,12 +547,12 @@ __device__ void control_warp(const IndexLaunch &P, PipeSmem<NT> &sm, const CUten
 }
 
 template <int LMAX, bool kTma, int NT>
-__device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, int s, uint32_t k,
+__device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, uint32_t k,
                                         RowState &st) {
   constexpr int NWARPS = NT / 32;
   constexpr uint64_t TILE_BYTES = uint64_t(NT) * 128u;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const StageMeta &m = sm.stage[s];
+  const StageMeta &m = sm.stage;
   const uint32_t tile = m.tile;
   const IndexFile F = m.F;
   const uint32_t ktile = tile - F.first_tile;
@@ -562,16 +565,16 @@ __device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
   const uint32_t lim = valid > row_byte ? valid - row_byte : 0u;
   const uint8_t *rp = P.in + F.in_off + byte0 + row_byte;
   uint32_t r[16];
-  if (row_in_smem) load_word_smem(sm.tiles[s], tid, 0, r);
+  if (row_in_smem) load_word_smem(sm.tile, tid, 0, r);
   else load_word_global(rp, lim, 0, r);
   const WordClasses c0 = classify64(r);
-  if (row_in_smem) load_word_smem(sm.tiles[s], tid, 1, r);
+  if (row_in_smem) load_word_smem(sm.tile, tid, 1, r);
   else load_word_global(rp, lim, 64, r);
   const WordClasses c1 = classify64(r);
   const uint32_t tp0 = trailing_escape_parity(c0.bs);
   const uint32_t tp1 = trailing_escape_parity(c1.bs);
   if (lane == 31) sm.last_tp[warp] = tp1;
-  compute_sync<NT>();  // (1) last_tp; every row of buffer s has been read
+  compute_sync<NT>();  // (1) last_tp; every row of the buffer has been read
   uint32_t cin0 = __shfl_up_sync(0xFFFFFFFFu, tp1, 1);
   if (lane == 0) cin0 = (warp == 0) ? m.halo : sm.last_tp[warp - 1];
 
@@ -629,25 +632,16 @@ __device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
     sm.warp_nl[warp] = nl_inc;
   }
   compute_sync<NT>();  // (3)
-  // inclusive scan of the warps' sums over lanes 0 .. NWARPS-1
-  uint32_t wdd = lane < NWARPS ? sm.warp_dd[lane < NWARPS ? lane : 0] : 0u;
-  uint32_t wnl = lane < NWARPS ? sm.warp_nl[lane < NWARPS ? lane : 0] : 0u;
-#pragma unroll
-  for (int off = 1; off < NWARPS; off <<= 1) {
-    const uint32_t a = __shfl_up_sync(0xFFFFFFFFu, wdd, off);
-    const uint32_t b = __shfl_up_sync(0xFFFFFFFFu, wnl, off);
-    if (lane >= off) {
-      wdd += a;
-      wnl += b;
-    }
+  // the warps' sums before this one; the first warp also needs their totals
+  const uint32_t wdd = lane < NWARPS ? sm.warp_dd[lane < NWARPS ? lane : 0] : 0u;
+  const uint32_t wnl = lane < NWARPS ? sm.warp_nl[lane < NWARPS ? lane : 0] : 0u;
+  const uint32_t dd_ex = dd_inc - dd + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? wdd : 0u);
+  const uint32_t nl_ex = nl_inc - thr_nl + __reduce_add_sync(0xFFFFFFFFu, lane < warp ? wnl : 0u);
+  uint32_t tile_dd = 0, tile_nl = 0;
+  if (warp == 0) {
+    tile_dd = __reduce_add_sync(0xFFFFFFFFu, wdd);
+    tile_nl = __reduce_add_sync(0xFFFFFFFFu, wnl);
   }
-  const int prev_warp = warp > 0 ? warp - 1 : 0;
-  const uint32_t before_dd = __shfl_sync(0xFFFFFFFFu, wdd, prev_warp);
-  const uint32_t before_nl = __shfl_sync(0xFFFFFFFFu, wnl, prev_warp);
-  const uint32_t tile_dd = __shfl_sync(0xFFFFFFFFu, wdd, NWARPS - 1);
-  const uint32_t tile_nl = __shfl_sync(0xFFFFFFFFu, wnl, NWARPS - 1);
-  const uint32_t dd_ex = dd_inc - dd + (warp > 0 ? before_dd : 0u);
-  const uint32_t nl_ex = nl_inc - thr_nl + (warp > 0 ? before_nl : 0u);
   if (tid == 0) {
     // publish the aggregate at once: look-backs of later tiles wait for it
     if (tile != 0)
@@ -892,19 +886,17 @@ __device__ __forceinline__ void phase_b(const IndexLaunch &P, PipeSmem<NT> &sm,
   }
   // newline offsets (every '\n' counts, strings or not), file-local
   uint64_t kk = nl_base;
-  uint64_t m = st.nl0;
-  while (m) {
+  uint64_t m0 = st.nl0, m1 = st.nl1;
+  while ((m0 | m1) != 0) {
+    const bool second = m0 == 0;
+    uint64_t m = second ? m1 : m0;
     const int b = __ffsll(static_cast<long long>(m)) - 1;
-    if (kk + 1 < P.nl_cap) P.NL[kk + 1] = int64_t(lw0 * 64u + uint64_t(b));
+    if (kk + 1 < P.nl_cap)
+      P.NL[kk + 1] = int64_t((lw0 + (second ? 1u : 0u)) * 64u + uint64_t(b));
     ++kk;
     m &= m - 1;
-  }
-  m = st.nl1;
-  while (m) {
-    const int b = __ffsll(static_cast<long long>(m)) - 1;
-    if (kk + 1 < P.nl_cap) P.NL[kk + 1] = int64_t((lw0 + 1) * 64u + uint64_t(b));
-    ++kk;
-    m &= m - 1;
+    if (second) m1 = m;
+    else m0 = m;
   }
 }
 
@@ -912,7 +904,7 @@ __device__ __forceinline__ void phase_b(const IndexLaunch &P, PipeSmem<NT> &sm,
 // threads; kList: the listed leveled walk; kLB: look-back descriptors per
 // lane; kPasses: more than LMAX levels, in passes.
 template <int LMAX, bool kTma, int NT, bool kList, int kLB, bool kPasses>
-__global__ void __launch_bounds__(NT + 32, NT <= 128 ? 4 : 2)
+__global__ void __launch_bounds__(NT + 32, NT <= 128 ? 5 : 3)
     index_kernel(const __grid_constant__ CUtensorMap tmap, const IndexLaunch P) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   // the 128-byte-swizzled TMA destinations need 1024-byte alignment
@@ -926,11 +918,8 @@ __global__ void __launch_bounds__(NT + 32, NT <= 128 ? 4 : 2)
   if (tid == NT) {
     // barriers must be initialised before anyone polls them: shared memory
     // may still hold barriers of an earlier CTA on this SM
-#pragma unroll
-    for (int s = 0; s < kStages; ++s) {
-      mbar_init(smem_u32(&sm.full[s]), 2);  // copy issued + escape carry written
-      sm.stage[s].tile = kEndTile;
-    }
+    mbar_init(smem_u32(&sm.full), 2);  // copy issued + escape carry written
+    sm.stage.tile = kEndTile;
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
       mbar_init(smem_u32(&sm.agg[j]), 1);
@@ -951,19 +940,18 @@ __global__ void __launch_bounds__(NT + 32, NT <= 128 ? 4 : 2)
   RowState prev{};
   uint32_t k = 0;
   for (;; ++k) {
-    const int s = int(k & 1u);
-    bool stop = !mbar_wait(smem_u32(&sm.full[s]), (k >> 1) & 1u, &sm.abort);
+    bool stop = !mbar_wait(smem_u32(&sm.full), k & 1u, &sm.abort);
     if (stop) {
       atomicOr(P.error, kErrTmaTimeout);
       sm.abort = 1;
     }
-    // one decision for all compute threads: buffer s is read only when every
+    // one decision for all compute threads: the buffer is read only when every
     // one of them saw it filled
     stop = compute_sync_or<NT>(stop || *static_cast<volatile uint32_t *>(&sm.abort) != 0 ||
-                               sm.stage[s].tile == kEndTile);
+                               sm.stage.tile == kEndTile);
     if (stop) break;
     RowState cur;
-    phase_a<LMAX, kTma, NT>(P, sm, s, k, cur);
+    phase_a<LMAX, kTma, NT>(P, sm, k, cur);
     if (k > 0) phase_b<LMAX, NT, kList, kPasses>(P, sm, ls, k - 1, prev);
     prev = cur;
   }
