@@ -104,9 +104,9 @@ bool host_range_mapped(const void *p, uint64_t bytes) {
   unsigned int type = 0;
   CUdeviceptr device = 0, start = 0;
   size_t size = 0;
-  CUpointer_attribute what[] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
-                                CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
-                                CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+  CUpointer_attribute what[] = {
+      CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_DEVICE_POINTER,
+      CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
   void *into[] = {&type, &device, &start, &size};
   const auto at = reinterpret_cast<CUdeviceptr>(p);
   if (get(4, what, into, at) != CUDA_SUCCESS) return false;

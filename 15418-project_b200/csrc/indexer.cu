@@ -288,7 +288,9 @@ __device__ __forceinline__ Agg tile_aggregate(uint32_t par, uint32_t dd, uint32_
 // spilled) put three CTAs of 256 threads on an SM: 1 GiB of products 566 ->
 // 528 us, of posts 591 -> 554 us against two CTAs with two buffers and 96
 // registers; three CTAs of 192 threads, with smaller tiles, were slower than
-// two of 256 (600 us).
+// two of 256 (600 us).  Phase A has two barriers: a warp reads the escape carry
+// of its first row from the staged tile itself, and the decision to stop rides
+// on the first barrier (four barriers: 528 and 554 us, now 518 and 544).
 //
 // Claiming just in time keeps the time from a tile's claim to its aggregate
 // the same for every CTA (phase B of one tile plus phase A of the next), so
@@ -337,7 +339,7 @@ struct PipeSmem {
   unsigned long long pref[2];
   StageMeta stage;
   TileMeta tm[2];
-  uint32_t last_tp[NW], warp_par[NW], warp_dd[NW], warp_nl[NW];
+  uint32_t warp_par[NW], warp_dd[NW], warp_nl[NW];
   uint32_t abort;
 };
 
@@ -546,68 +548,101 @@ __device__ void control_warp(const IndexLaunch &P, PipeSmem<NT> &sm, const CUten
   }
 }
 
+// Parity of the backslash run that ends the row before the calling thread's
+// (the first row of a warp): the carry of trailing_escape_parity, read back
+// from the staged tile, or from the input where that row is not staged.
+template <bool kTma>
+__device__ __forceinline__ uint32_t escape_parity_before(const uint8_t *tile, uint32_t row,
+                                                         uint32_t smem_rows, const uint8_t *rp,
+                                                         uint32_t valid) {
+  const uint32_t prev = row - 1u;
+  uint32_t run = 0;
+  if (kTma && prev < smem_rows) {
+    const uint8_t *base = tile + prev * 128u;
+    while (run < 64u) {
+      const uint32_t at = 127u - run;
+      if (base[(((at >> 4) ^ (prev & 7u)) << 4) + (at & 15u)] != '\\') break;
+      ++run;
+    }
+  } else if (valid >= row * 128u) {  // else the file ended before this row
+    while (run < 64u && rp[-1 - int(run)] == '\\') ++run;
+  }
+  return run & 1u;
+}
+
+// Phase A of the staged tile.  `stop` (the same for all lanes of a warp): this
+// warp gave up or the CTA has no more tiles.  Returns false when any compute
+// warp stopped, without a trace of the tile.
 template <int LMAX, bool kTma, int NT>
-__device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, uint32_t k,
-                                        RowState &st) {
+__device__ __forceinline__ bool phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, uint32_t k,
+                                        bool stop, RowState &st) {
   constexpr int NWARPS = NT / 32;
   constexpr uint64_t TILE_BYTES = uint64_t(NT) * 128u;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const StageMeta &m = sm.stage;
-  const uint32_t tile = m.tile;
-  const IndexFile F = m.F;
-  const uint32_t ktile = tile - F.first_tile;
-  const uint64_t byte0 = uint64_t(ktile) * TILE_BYTES;
-  const uint32_t valid = m.valid;
-  const uint32_t row_byte = uint32_t(tid) * 128u;
-  const uint64_t lw0 = byte0 / 64u + 2u * uint64_t(tid);
-  const bool row_in_smem = kTma && uint32_t(tid) < m.smem_rows;
-  // rows past the end of the file read as zero bytes (no class)
-  const uint32_t lim = valid > row_byte ? valid - row_byte : 0u;
-  const uint8_t *rp = P.in + F.in_off + byte0 + row_byte;
-  uint32_t r[16];
-  if (row_in_smem) load_word_smem(sm.tile, tid, 0, r);
-  else load_word_global(rp, lim, 0, r);
-  const WordClasses c0 = classify64(r);
-  if (row_in_smem) load_word_smem(sm.tile, tid, 1, r);
-  else load_word_global(rp, lim, 64, r);
-  const WordClasses c1 = classify64(r);
-  const uint32_t tp0 = trailing_escape_parity(c0.bs);
-  const uint32_t tp1 = trailing_escape_parity(c1.bs);
-  if (lane == 31) sm.last_tp[warp] = tp1;
-  compute_sync<NT>();  // (1) last_tp; every row of the buffer has been read
-  uint32_t cin0 = __shfl_up_sync(0xFFFFFFFFu, tp1, 1);
-  if (lane == 0) cin0 = (warp == 0) ? m.halo : sm.last_tp[warp - 1];
+  WordClasses c0, c1;
+  uint64_t Sl0 = 0, Sl1 = 0;
+  uint32_t par0 = 0, thr_par = 0, par_ballot = 0, thr_nl = 0;
+  int thr_d0 = 0, thr_t = 0;
+  if (!stop) {
+    const IndexFile F = m.F;
+    const uint32_t ktile = m.tile - F.first_tile;
+    const uint64_t byte0 = uint64_t(ktile) * TILE_BYTES;
+    const uint32_t valid = m.valid;
+    const uint32_t row_byte = uint32_t(tid) * 128u;
+    const uint64_t lw0 = byte0 / 64u + 2u * uint64_t(tid);
+    const bool row_in_smem = kTma && uint32_t(tid) < m.smem_rows;
+    // rows past the end of the file read as zero bytes (no class)
+    const uint32_t lim = valid > row_byte ? valid - row_byte : 0u;
+    const uint8_t *rp = P.in + F.in_off + byte0 + row_byte;
+    uint32_t r[16];
+    if (row_in_smem) load_word_smem(sm.tile, tid, 0, r);
+    else load_word_global(rp, lim, 0, r);
+    c0 = classify64(r);
+    if (row_in_smem) load_word_smem(sm.tile, tid, 1, r);
+    else load_word_global(rp, lim, 64, r);
+    c1 = classify64(r);
+    const uint32_t tp0 = trailing_escape_parity(c0.bs);
+    const uint32_t tp1 = trailing_escape_parity(c1.bs);
+    uint32_t cin0 = __shfl_up_sync(0xFFFFFFFFu, tp1, 1);
+    if (lane == 0)
+      cin0 = warp == 0
+                 ? m.halo
+                 : escape_parity_before<kTma>(sm.tile, uint32_t(tid), m.smem_rows, rp, valid);
 
-  const uint64_t E0 = escaped_bits(c0.bs, cin0);
-  const uint64_t E1 = escaped_bits(c1.bs, tp0);
-  const uint64_t Q0 = c0.qt & ~E0;
-  const uint64_t Q1 = c1.qt & ~E1;
-  const uint64_t Sl0 = prefix_xor(Q0);
-  const uint64_t Sl1 = prefix_xor(Q1);
-  // a word's quote parity is the top bit of its in-word prefix-XOR
-  const uint32_t par0 = uint32_t(Sl0 >> 63);
-  const uint32_t par1 = uint32_t(Sl1 >> 63);
-  if (P.E != nullptr) {
-    const uint64_t W = (F.n + 63u) / 64u;
-    store2(P.E + F.s_off, lw0, W, E0 & valid_mask(lw0, F.n), E1 & valid_mask(lw0 + 1, F.n));
-    store2(P.Q + F.s_off, lw0, W, Q0, Q1);
+    const uint64_t E0 = escaped_bits(c0.bs, cin0);
+    const uint64_t E1 = escaped_bits(c1.bs, tp0);
+    const uint64_t Q0 = c0.qt & ~E0;
+    const uint64_t Q1 = c1.qt & ~E1;
+    Sl0 = prefix_xor(Q0);
+    Sl1 = prefix_xor(Q1);
+    // a word's quote parity is the top bit of its in-word prefix-XOR
+    par0 = uint32_t(Sl0 >> 63);
+    const uint32_t par1 = uint32_t(Sl1 >> 63);
+    if (P.E != nullptr) {
+      const uint64_t W = (F.n + 63u) / 64u;
+      store2(P.E + F.s_off, lw0, W, E0 & valid_mask(lw0, F.n), E1 & valid_mask(lw0 + 1, F.n));
+      store2(P.Q + F.s_off, lw0, W, Q0, Q1);
+    }
+
+    // depth change of each word if it starts outside a string, and in total
+    const int d00 = popc64(c0.op & ~Sl0) - popc64(c0.cl & ~Sl0);
+    const int t0 = popc64(c0.op) - popc64(c0.cl);
+    const int d10 = popc64(c1.op & ~Sl1) - popc64(c1.cl & ~Sl1);
+    const int t1 = popc64(c1.op) - popc64(c1.cl);
+    thr_d0 = d00 + (par0 ? (t1 - d10) : d10);
+    thr_t = t0 + t1;
+    thr_par = par0 ^ par1;
+    thr_nl = uint32_t(popc64(c0.nl) + popc64(c1.nl));
+
+    par_ballot = __ballot_sync(0xFFFFFFFFu, thr_par);
+    if (lane == 0) sm.warp_par[warp] = uint32_t(__popc(par_ballot)) & 1u;
   }
-
-  // depth change of each word if it starts outside a string, and in total
-  const int d00 = popc64(c0.op & ~Sl0) - popc64(c0.cl & ~Sl0);
-  const int t0 = popc64(c0.op) - popc64(c0.cl);
-  const int d10 = popc64(c1.op & ~Sl1) - popc64(c1.cl & ~Sl1);
-  const int t1 = popc64(c1.op) - popc64(c1.cl);
-  const int thr_d0 = d00 + (par0 ? (t1 - d10) : d10);
-  const int thr_t = t0 + t1;
-  const uint32_t thr_par = par0 ^ par1;
-  const uint32_t thr_nl = uint32_t(popc64(c0.nl) + popc64(c1.nl));
-
+  // (1) the warps' parities; every row of the buffer has been read; one
+  // decision for all compute threads whether the tile stands
+  if (compute_sync_or<NT>(stop)) return false;
   const uint32_t lt_mask = (1u << lane) - 1u;
-  const uint32_t par_ballot = __ballot_sync(0xFFFFFFFFu, thr_par);
   uint32_t pex = uint32_t(__popc(par_ballot & lt_mask)) & 1u;
-  if (lane == 0) sm.warp_par[warp] = uint32_t(__popc(par_ballot)) & 1u;
-  compute_sync<NT>();  // (2)
   // the warps' parities as one bit mask (lane w reads warp w's)
   const uint32_t wpar =
       __ballot_sync(0xFFFFFFFFu, lane < NWARPS && sm.warp_par[lane < NWARPS ? lane : 0] != 0u);
@@ -631,7 +666,7 @@ __device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
     sm.warp_dd[warp] = dd_inc;
     sm.warp_nl[warp] = nl_inc;
   }
-  compute_sync<NT>();  // (3)
+  compute_sync<NT>();  // (2)
   // the warps' sums before this one; the first warp also needs their totals
   const uint32_t wdd = lane < NWARPS ? sm.warp_dd[lane < NWARPS ? lane : 0] : 0u;
   const uint32_t wnl = lane < NWARPS ? sm.warp_nl[lane < NWARPS ? lane : 0] : 0u;
@@ -644,6 +679,10 @@ __device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
   }
   if (tid == 0) {
     // publish the aggregate at once: look-backs of later tiles wait for it
+    const uint32_t tile = m.tile;
+    const IndexFile F = m.F;
+    const uint32_t ktile = tile - F.first_tile;
+    const uint64_t byte0 = uint64_t(ktile) * TILE_BYTES;
     if (tile != 0)
       st_relaxed(&P.tile_state[tile],
                  agg_pack(kStatusAgg, tile_aggregate(tile_par, tile_dd, tile_nl, ktile == 0)));
@@ -686,6 +725,7 @@ __device__ __forceinline__ void phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
   st.par0 = par0;
   st.dd_ex = dd_ex;
   st.nl_ex = nl_ex;
+  return true;
 }
 
 // Leveled bitmaps of one lane's two words, walked as event sequences in
@@ -945,13 +985,10 @@ __global__ void __launch_bounds__(NT + 32, NT <= 128 ? 5 : 3)
       atomicOr(P.error, kErrTmaTimeout);
       sm.abort = 1;
     }
-    // one decision for all compute threads: the buffer is read only when every
-    // one of them saw it filled
-    stop = compute_sync_or<NT>(stop || *static_cast<volatile uint32_t *>(&sm.abort) != 0 ||
-                               sm.stage.tile == kEndTile);
-    if (stop) break;
+    stop = __any_sync(0xFFFFFFFFu, stop || *static_cast<volatile uint32_t *>(&sm.abort) != 0 ||
+                                       sm.stage.tile == kEndTile);
     RowState cur;
-    phase_a<LMAX, kTma, NT>(P, sm, k, cur);
+    if (!phase_a<LMAX, kTma, NT>(P, sm, k, stop, cur)) break;
     if (k > 0) phase_b<LMAX, NT, kList, kPasses>(P, sm, ls, k - 1, prev);
     prev = cur;
   }
@@ -1019,12 +1056,12 @@ template <int NT>
 cudaError_t launch_threads(const IndexLaunch &L, const CUtensorMap *map, bool use_tma,
                            bool overlap, cudaStream_t stream) {
   const int lv = L.num_levels;
-  if (lv <= 2) return launch_levels<2, NT>(L, map, use_tma, overlap, stream);
   if (lv <= 4) return launch_levels<4, NT>(L, map, use_tma, overlap, stream);
-  if (lv <= kSharedLevels) return launch_levels<kSharedLevels, NT>(L, map, use_tma, overlap, stream);
-  // 96 MiB of posts: 8 levels 81 us; in passes 12, 15 and 22 levels 103, 104
-  // and 111 us (191, 193 and 197 us in an instance that held 22 levels in
-  // registers and went over all of them at every bracket)
+  if (lv <= kSharedLevels)
+    return launch_levels<kSharedLevels, NT>(L, map, use_tma, overlap, stream);
+  // 96 MiB of posts: 8 levels 69 us; in passes 15 levels 93 us (193 us in an
+  // instance that held 22 levels in registers and went over all of them at
+  // every bracket)
   return launch_tma<kSharedLevels, NT, false, 1, true>(L, map, use_tma, overlap, stream);
 }
 
