@@ -1033,8 +1033,9 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
 // kExt: the IR holds extension opcodes (numeric filters, "..name", the
 // element checks of "[*]" and the open slices); reference-syntax IR runs the
 // variant without them.
-template <typename Pos, typename OutT, bool kExt, int G>
-__global__ void __launch_bounds__(256, sizeof(Pos) == 8 ? 3 : (G == 1 ? 5 : 4))
+// kBlocks: 256-thread blocks per SM that the registers are held to.
+template <typename Pos, typename OutT, bool kExt, int G, int kBlocks>
+__global__ void __launch_bounds__(256, kBlocks)
     query_kernel(const QueryLaunch q, const __grid_constant__ IrBlob ir, OutT *out, int nlev) {
   __shared__ __align__(16) uint8_t s_ir[kMaxQueryIrBytes + kIrPad];
   extern __shared__ __align__(8) uint8_t s_state[];  // Pos[nlev + marks][bdim]
@@ -1343,7 +1344,7 @@ void batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, bool ext, in
   else batch_query_kernel<false, G><<<grid, block, smem, stream>>>(q, ir, nlev);
 }
 
-template <typename Pos, typename OutT, int G>
+template <typename Pos, typename OutT, int G, int kBlocks>
 void query_start(const QueryLaunch &q, const IrBlob &ir, OutT *out, int grid, int block,
                  cudaStream_t stream) {
   if (grid <= 0) {
@@ -1354,18 +1355,44 @@ void query_start(const QueryLaunch &q, const IrBlob &ir, OutT *out, int grid, in
   const size_t smem =
       size_t(nlev + query_ir_marks(ir.bytes, q.ir_len)) * size_t(block) * sizeof(Pos);
   if (query_ir_uses_extensions(ir.bytes, q.ir_len))
-    query_kernel<Pos, OutT, true, G><<<grid, block, smem, stream>>>(q, ir, out, nlev);
+    query_kernel<Pos, OutT, true, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, out, nlev);
   else
-    query_kernel<Pos, OutT, false, G><<<grid, block, smem, stream>>>(q, ir, out, nlev);
+    query_kernel<Pos, OutT, false, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, out, nlev);
+}
+
+// Blocks per SM of the one-lane kernel.  Its blocks start together and take
+// about as long as each other, so a launch runs in waves, and a wave takes time
+// in proportion to the blocks of it per SM from four on ($.user.lang on posts:
+// 76, 98 and 126 us for a full wave of four, five and six): the fewest waves
+// times blocks win, fewer blocks where two are equal.  153 K array elements:
+// 87, 71 and 78 us with four, five and six; 208 K: 111, 124 and 102; 236 K:
+// 113, 128 and 160; 349 K: 165, 145 and 182.
+int blocks_per_sm(uint64_t records) {
+  const uint64_t per_block = resident_threads() / 4u;  // one block on every SM
+  int best = 4;
+  uint64_t best_cost = ~uint64_t(0);
+  for (int b : {4, 5, 6}) {
+    const uint64_t wave = per_block * uint64_t(b);
+    const uint64_t cost = (records + wave - 1) / wave * uint64_t(b);
+    if (cost < best_cost) {
+      best = b;
+      best_cost = cost;
+    }
+  }
+  return best;
 }
 
 template <typename OutT>
 void query_start_narrow(const QueryLaunch &q, const IrBlob &ir, OutT *out, int lanes, int grid,
                         int block, cudaStream_t stream) {
-  if (lanes == 32) query_start<int32_t, OutT, 32>(q, ir, out, grid, block, stream);
-  else if (lanes == 16) query_start<int32_t, OutT, 16>(q, ir, out, grid, block, stream);
-  else if (lanes == 8) query_start<int32_t, OutT, 8>(q, ir, out, grid, block, stream);
-  else query_start<int32_t, OutT, 1>(q, ir, out, grid, block, stream);
+  if (lanes == 32) return query_start<int32_t, OutT, 32, 4>(q, ir, out, grid, block, stream);
+  if (lanes == 16) return query_start<int32_t, OutT, 16, 4>(q, ir, out, grid, block, stream);
+  if (lanes == 8) return query_start<int32_t, OutT, 8, 4>(q, ir, out, grid, block, stream);
+  switch (blocks_per_sm(uint64_t(q.num_lines))) {
+  case 5: return query_start<int32_t, OutT, 1, 5>(q, ir, out, grid, block, stream);
+  case 6: return query_start<int32_t, OutT, 1, 6>(q, ir, out, grid, block, stream);
+  default: return query_start<int32_t, OutT, 1, 4>(q, ir, out, grid, block, stream);
+  }
 }
 
 }  // namespace
@@ -1413,9 +1440,9 @@ cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, int grid,
   else if (q.n <= 0x7FFFFFFF)
     query_start_narrow(q, ir, q.out64, lanes, grid, block, stream);
   else if (lanes == 32)
-    query_start<int64_t, int64_t, 32>(q, ir, q.out64, grid, block, stream);
+    query_start<int64_t, int64_t, 32, 3>(q, ir, q.out64, grid, block, stream);
   else
-    query_start<int64_t, int64_t, 1>(q, ir, q.out64, grid, block, stream);
+    query_start<int64_t, int64_t, 1, 3>(q, ir, q.out64, grid, block, stream);
   return cudaGetLastError();
 }
 

@@ -132,3 +132,29 @@ def test_every_split_of_a_batch_matches_oracle(gpj, end):
             want = oracle.OracleIndex(np.frombuffer(f, np.uint8), c.max_depth).query(
                 c.ir_bytes, c.num_result_slots)
             np.testing.assert_array_equal(res.astype(np.int64), want, err_msg=c.query_text)
+
+
+@pytest.mark.parametrize("blocks", [4, 5, 6])
+@pytest.mark.parametrize("query", ["$.key.ab", "$.arr[*]"])
+def test_one_lane_at_every_block_count(cuda_ctx, gpj, blocks, query):
+    """One lane per record in launches of one full wave of 4, 5 or 6 blocks per
+    SM, plus the records of a half block."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    count = sms * 256 * blocks - 128
+    part = _lines(77, 20000)
+    data = np.frombuffer(b"\n".join([part] * (count // 20000 + 1)), np.uint8)
+    ends = np.flatnonzero(data == 10)
+    data = data[: int(ends[count - 1])]
+    c = gpj.compile(query, wildcard_limit=4)
+    buf = torch.from_numpy(data.copy()).cuda()
+    ix = cuda_ctx.build_index(buf.data_ptr(), data.size, c.max_depth)
+    try:
+        assert ix.num_lines == count
+        out = torch.full((count, c.num_result_slots, 2), -7, dtype=torch.int32, device="cuda")
+        cuda_ctx.query(ix, c, out.data_ptr())
+        torch.cuda.synchronize()
+        cuda_ctx.query_status()
+        want = oracle.OracleIndex(data, c.max_depth).query(c.ir_bytes, c.num_result_slots)
+        np.testing.assert_array_equal(out.cpu().numpy().astype(np.int64), want)
+    finally:
+        cuda_ctx.free_index(ix)
