@@ -485,15 +485,12 @@ int gpj_batch_run_per_file(gpj_batch *b, void *stream_) {
     q.S = L.S;
     q.LB = L.LB;
     q.W = int64_t((F.n + 63u) / 64u);
-    q.ir_len = G.ir_len;
-    q.num_results = G.num_results;
     q.num_levels = F.levels;
-    q.base_level = G.base_level;
-    q.out32 = b->d_out + row[gpjb::kFiOutOff];
+    q.queries[0] = {0, G.ir_len, G.num_results, G.base_level, b->d_out + row[gpjb::kFiOutOff]};
     q.status = reinterpret_cast<unsigned int *>(b->d_totals + gpjb::kTotError);
     gpjb::IrBlob blob;
     std::memcpy(blob.bytes, b->blob.bytes + G.ir_off, size_t(G.ir_len));
-    BCUDA(gpjb::query_launch(q, blob, 0, 256, stream), "per-file query launch");
+    BCUDA(gpjb::query_launch(q, blob, stream), "per-file query launch");
   }
   return GPJ_OK;
 }

@@ -417,43 +417,72 @@ int check_levels(int levels) {
   return GPJ_OK;
 }
 
+// One query of a run: its IR and where its results go.
+struct QueryRun {
+  const uint8_t *h_ir;
+  uint64_t ir_len;
+  uint32_t slots, base_level;
+  void *d_out;
+};
+
+// Checks the queries one after another and launches them: as many together as
+// one launch takes (a launch of one query leaves most of the device idle on
+// small partitions).
+int run_queries(gpj_ctx *ctx, const gpj_index *ix, const QueryRun *runs, size_t count, bool wide,
+                cudaStream_t stream) {
+  gpjb::QueryLaunch q;
+  gpjb::IrBlob blob;
+  int ir_bytes = 0;
+  q.num_queries = 0;
+  auto flush = [&]() -> int {
+    if (q.num_queries == 0) return GPJ_OK;
+    GPJ_CUDA(gpjb::query_launch(q, blob, stream), "query kernel launch");
+    q.num_queries = 0;
+    ir_bytes = 0;
+    return GPJ_OK;
+  };
+  for (size_t i = 0; i < count; ++i) {
+    const QueryRun &r = runs[i];
+    if (ix == nullptr || r.d_out == nullptr || r.h_ir == nullptr)
+      return fail(GPJ_ERR_INVALID_ARGUMENT, "null argument");
+    if (r.ir_len > uint64_t(GPJ_MAX_QUERY_IR))
+      return fail(GPJ_ERR_EXECUTION, "Compiled query IR exceeds constant memory buffer");
+    if (ix->num_lines == 0 || ix->size_bytes == 0) continue;
+    if (ix->num_lines > ix->newline_capacity)
+      return fail(GPJ_ERR_CAPACITY, "newline index was truncated: rebuild with capacity >= " +
+                                        std::to_string(ix->num_lines));
+    if (r.base_level > 0 && int64_t(r.base_level) >= int64_t(ix->num_levels))
+      return fail(GPJ_ERR_EXECUTION, "Query requires more bitmap levels than the index provides");
+    if (!wide && ix->size_bytes > 0x7FFFFFFFull)
+      return fail(GPJ_ERR_EXECUTION, "partition size exceeds CUDA int range");
+    int rc = bind_device(ctx);
+    if (rc == GPJ_OK && (q.num_queries == gpjb::kMaxLaunchQueries ||
+                         ir_bytes + int(r.ir_len) > gpjb::kMaxQueryIrBytes))
+      rc = flush();
+    if (rc != GPJ_OK) return rc;
+    q.in = ix->d_input;
+    q.n = int64_t(ix->size_bytes);
+    q.NL = ix->d_newline;
+    q.num_lines = int64_t(ix->num_lines);
+    q.S = ix->d_string;
+    q.LB = ix->d_leveled;
+    q.W = int64_t(ix->num_words);
+    q.num_levels = ix->num_levels;
+    q.wide = wide;
+    q.status = ctx->d_status;
+    q.queries[q.num_queries++] = {ir_bytes, int(r.ir_len), int(r.slots), int(r.base_level),
+                                  r.d_out};
+    std::memcpy(blob.bytes + ir_bytes, r.h_ir, size_t(r.ir_len));
+    ir_bytes += int(r.ir_len);
+  }
+  return flush();
+}
+
 template <typename OutT>
 int run_query(gpj_ctx *ctx, const gpj_index *ix, const uint8_t *h_ir, uint64_t ir_len,
               uint32_t slots, OutT *d_out, cudaStream_t stream, uint32_t base_level = 0) {
-  if (ix == nullptr || d_out == nullptr || h_ir == nullptr)
-    return fail(GPJ_ERR_INVALID_ARGUMENT, "null argument");
-  if (ir_len > uint64_t(GPJ_MAX_QUERY_IR))
-    return fail(GPJ_ERR_EXECUTION, "Compiled query IR exceeds constant memory buffer");
-  if (ix->num_lines == 0 || ix->size_bytes == 0) return GPJ_OK;
-  if (ix->num_lines > ix->newline_capacity)
-    return fail(GPJ_ERR_CAPACITY, "newline index was truncated: rebuild with capacity >= " +
-                                      std::to_string(ix->num_lines));
-  if (base_level > 0 && int64_t(base_level) >= int64_t(ix->num_levels))
-    return fail(GPJ_ERR_EXECUTION, "Query requires more bitmap levels than the index provides");
-  if (sizeof(OutT) == 4 && ix->size_bytes > 0x7FFFFFFFull)
-    return fail(GPJ_ERR_EXECUTION, "partition size exceeds CUDA int range");
-  int rc = bind_device(ctx);
-  if (rc != GPJ_OK) return rc;
-  gpjb::QueryLaunch q;
-  q.in = ix->d_input;
-  q.n = int64_t(ix->size_bytes);
-  q.NL = ix->d_newline;
-  q.num_lines = int64_t(ix->num_lines);
-  q.S = ix->d_string;
-  q.LB = ix->d_leveled;
-  q.W = int64_t(ix->num_words);
-  q.ir_len = int(ir_len);
-  q.num_results = int(slots);
-  q.base_level = int(base_level);
-  q.num_levels = ix->num_levels;
-  if constexpr (sizeof(OutT) == 8) q.out64 = reinterpret_cast<int64_t *>(d_out);
-  else q.out32 = reinterpret_cast<int32_t *>(d_out);
-  q.status = ctx->d_status;
-  gpjb::IrBlob blob;
-  std::memset(blob.bytes, 0, sizeof(blob.bytes));
-  std::memcpy(blob.bytes, h_ir, size_t(ir_len));
-  GPJ_CUDA(gpjb::query_launch(q, blob, 0, 256, stream), "query kernel launch");
-  return GPJ_OK;
+  const QueryRun run{h_ir, ir_len, slots, base_level, d_out};
+  return run_queries(ctx, ix, &run, 1, sizeof(OutT) == 8, stream);
 }
 
 }  // namespace
@@ -725,17 +754,21 @@ int gpj_query_host(gpj_ctx *ctx, const uint8_t *h_input, uint64_t size_bytes, in
     rc = ensure(ctx->host_results, ctx->host_results_bytes, total);
     if (rc != GPJ_OK) return rc;
     GPJ_CUDA(cudaMemsetAsync(ctx->d_status, 0, 4, stream), "clear status");
+    std::vector<QueryRun> runs;
     uint64_t off = 0;
     for (uint32_t q = 0; q < num_queries; ++q) {
-      auto *d_out = reinterpret_cast<int32_t *>(static_cast<unsigned char *>(ctx->host_results) + off);
-      rc = run_query<int32_t>(ctx, &ix, h_irs[q], ir_lens[q], num_result_slots[q], d_out, stream,
-                              base_levels ? base_levels[q] : 0u);
-      if (rc != GPJ_OK) return rc;
-      const uint64_t need = lines * uint64_t(num_result_slots[q]) * 2u;
-      if (need > 0)
-        GPJ_CUDA(cudaMemcpyAsync(h_out[q], d_out, need * 4u, cudaMemcpyDeviceToHost, stream),
+      runs.push_back({h_irs[q], ir_lens[q], num_result_slots[q],
+                      base_levels ? base_levels[q] : 0u,
+                      static_cast<unsigned char *>(ctx->host_results) + off});
+      off += round256(lines * uint64_t(num_result_slots[q]) * 8u);
+    }
+    rc = run_queries(ctx, &ix, runs.data(), runs.size(), false, stream);
+    if (rc != GPJ_OK) return rc;
+    for (uint32_t q = 0; q < num_queries; ++q) {
+      const uint64_t bytes = lines * uint64_t(num_result_slots[q]) * 8u;
+      if (bytes > 0)
+        GPJ_CUDA(cudaMemcpyAsync(h_out[q], runs[q].d_out, bytes, cudaMemcpyDeviceToHost, stream),
                  "copy results");
-      off += round256(need * 4u);
     }
     auto *h_status = reinterpret_cast<unsigned int *>(ctx->pinned + 6);
     GPJ_CUDA(cudaMemcpyAsync(h_status, ctx->d_status, 4, cudaMemcpyDeviceToHost, stream),

@@ -1036,17 +1036,20 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
 // kBlocks: 256-thread blocks per SM that the registers are held to.
 template <typename Pos, typename OutT, bool kExt, int G, int kBlocks>
 __global__ void __launch_bounds__(256, kBlocks)
-    query_kernel(const QueryLaunch q, const __grid_constant__ IrBlob ir, OutT *out, int nlev) {
+    query_kernel(const __grid_constant__ QueryLaunch q, const __grid_constant__ IrBlob ir,
+                 int nlev) {
   __shared__ __align__(16) uint8_t s_ir[kMaxQueryIrBytes + kIrPad];
-  extern __shared__ __align__(8) uint8_t s_state[];  // Pos[nlev + marks][bdim]
-  for (int i = threadIdx.x; i < q.ir_len + kIrPad; i += blockDim.x)
-    s_ir[i] = i < q.ir_len ? ir.bytes[i] : uint8_t(0);
-  __syncthreads();
   __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed<G>];
   __shared__ Pos s_match[kExt && G == 32 ? 8 : 1][32];
+  extern __shared__ __align__(8) uint8_t s_state[];  // Pos[nlev + marks][bdim]
+  const QueryOne &one = q.queries[blockIdx.y];
+  for (int i = threadIdx.x; i < one.ir_len + kIrPad; i += blockDim.x)
+    s_ir[i] = i < one.ir_len ? ir.bytes[one.ir_off + i] : uint8_t(0);
+  __syncthreads();
   const Group<G> g;
   const Rec<Pos> c{q.in, Pos(q.n), q.S, q.LB, Pos(q.W), q.num_levels, q.status};
-  const Query query{s_ir, q.ir_len, q.num_results, q.base_level, nlev};
+  const Query query{s_ir, one.ir_len, one.num_results, one.base_level, nlev};
+  OutT *const out = static_cast<OutT *>(one.out);
   Pos *ends = reinterpret_cast<Pos *>(s_state) + threadIdx.x;
   Pos *marks = ends + nlev * blockDim.x;
   const int64_t warps = int64_t(blockDim.x / 32u) * gridDim.x;
@@ -1057,9 +1060,9 @@ __global__ void __launch_bounds__(256, kBlocks)
     const int64_t start = alive ? q.NL[r] : 0;
     const int64_t end = alive && r + 1 < q.num_lines ? q.NL[r + 1] : q.n - 1;
     run_records<Pos, OutT, kExt, G>(c, query, g, alive, Pos(start), Pos(end),
-                                    out + r * int64_t(q.num_results) * 2, ends, marks,
+                                    out + r * int64_t(one.num_results) * 2, ends, marks,
                                     int(blockDim.x), s_list[G > 1 ? threadIdx.x / G : 0],
-            s_match[kExt && G == 32 ? threadIdx.x / 32 : 0]);
+                                    s_match[kExt && G == 32 ? threadIdx.x / 32 : 0]);
     __syncwarp();
   }
 }
@@ -1344,20 +1347,30 @@ void batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, bool ext, in
   else batch_query_kernel<false, G><<<grid, block, smem, stream>>>(q, ir, nlev);
 }
 
-template <typename Pos, typename OutT, int G, int kBlocks>
-void query_start(const QueryLaunch &q, const IrBlob &ir, OutT *out, int grid, int block,
-                 cudaStream_t stream) {
-  if (grid <= 0) {
-    const int64_t per_block = block / G;
-    grid = int(std::min<int64_t>((q.num_lines + per_block - 1) / per_block, 0x7FFFFFFF));
+// What the queries of a launch need together.
+struct QueryNeeds {
+  int nlev = 1, marks = 0;
+  bool ext = false, descends = false;
+  void add(const uint8_t *ir, int len) {
+    nlev = std::max(nlev, query_ir_levels(ir, len));
+    marks = std::max(marks, query_ir_marks(ir, len));
+    ext = ext || query_ir_uses_extensions(ir, len);
+    descends = descends || query_ir_descends(ir, len);
   }
-  const int nlev = query_ir_levels(ir.bytes, q.ir_len);
-  const size_t smem =
-      size_t(nlev + query_ir_marks(ir.bytes, q.ir_len)) * size_t(block) * sizeof(Pos);
-  if (query_ir_uses_extensions(ir.bytes, q.ir_len))
-    query_kernel<Pos, OutT, true, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, out, nlev);
+};
+
+template <typename Pos, typename OutT, int G, int kBlocks>
+void query_start(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs, int block,
+                 cudaStream_t stream) {
+  const int64_t per_block = block / G;
+  const dim3 grid(
+      unsigned(std::min<int64_t>((q.num_lines + per_block - 1) / per_block, 0x7FFFFFFF)),
+      unsigned(q.num_queries));
+  const size_t smem = size_t(needs.nlev + needs.marks) * size_t(block) * sizeof(Pos);
+  if (needs.ext)
+    query_kernel<Pos, OutT, true, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, needs.nlev);
   else
-    query_kernel<Pos, OutT, false, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, out, nlev);
+    query_kernel<Pos, OutT, false, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, needs.nlev);
 }
 
 // Blocks per SM of the one-lane kernel.  Its blocks start together and take
@@ -1383,15 +1396,15 @@ int blocks_per_sm(uint64_t records) {
 }
 
 template <typename OutT>
-void query_start_narrow(const QueryLaunch &q, const IrBlob &ir, OutT *out, int lanes, int grid,
-                        int block, cudaStream_t stream) {
-  if (lanes == 32) return query_start<int32_t, OutT, 32, 4>(q, ir, out, grid, block, stream);
-  if (lanes == 16) return query_start<int32_t, OutT, 16, 4>(q, ir, out, grid, block, stream);
-  if (lanes == 8) return query_start<int32_t, OutT, 8, 4>(q, ir, out, grid, block, stream);
-  switch (blocks_per_sm(uint64_t(q.num_lines))) {
-  case 5: return query_start<int32_t, OutT, 1, 5>(q, ir, out, grid, block, stream);
-  case 6: return query_start<int32_t, OutT, 1, 6>(q, ir, out, grid, block, stream);
-  default: return query_start<int32_t, OutT, 1, 4>(q, ir, out, grid, block, stream);
+void query_start_narrow(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs, int lanes,
+                        uint64_t runs, int block, cudaStream_t stream) {
+  if (lanes == 32) return query_start<int32_t, OutT, 32, 4>(q, ir, needs, block, stream);
+  if (lanes == 16) return query_start<int32_t, OutT, 16, 4>(q, ir, needs, block, stream);
+  if (lanes == 8) return query_start<int32_t, OutT, 8, 4>(q, ir, needs, block, stream);
+  switch (blocks_per_sm(runs)) {
+  case 5: return query_start<int32_t, OutT, 1, 5>(q, ir, needs, block, stream);
+  case 6: return query_start<int32_t, OutT, 1, 6>(q, ir, needs, block, stream);
+  default: return query_start<int32_t, OutT, 1, 4>(q, ir, needs, block, stream);
   }
 }
 
@@ -1399,50 +1412,44 @@ void query_start_narrow(const QueryLaunch &q, const IrBlob &ir, OutT *out, int l
 
 cudaError_t batch_query_launch(const BatchQueryLaunch &q, const IrBlob &ir, int grid,
                                int block, cudaStream_t stream) {
-  int nlev = 1, marks = 0;
-  bool ext = false, descends = false;
-  for (int g = 0; g < q.num_groups; ++g) {
-    const uint8_t *bytes = ir.bytes + q.groups[g].ir_off;
-    const int len = q.groups[g].ir_len;
-    nlev = std::max(nlev, query_ir_levels(bytes, len));
-    marks = std::max(marks, query_ir_marks(bytes, len));
-    ext = ext || query_ir_uses_extensions(bytes, len);
-    descends = descends || query_ir_descends(bytes, len);
-  }
-  const int lanes = lanes_per_record(q.expected_records, descends);
+  QueryNeeds needs;
+  for (int g = 0; g < q.num_groups; ++g)
+    needs.add(ir.bytes + q.groups[g].ir_off, q.groups[g].ir_len);
+  const int lanes = lanes_per_record(q.expected_records, needs.descends);
   if (q.expected_records > 0) {
     const uint64_t blocks = (q.expected_records * uint64_t(lanes) + uint64_t(block) - 1) / block;
     grid = int(std::min<uint64_t>(uint64_t(grid), blocks));
   }
-  const size_t smem = size_t(nlev + marks) * size_t(block) * sizeof(int32_t);
+  const size_t smem = size_t(needs.nlev + needs.marks) * size_t(block) * sizeof(int32_t);
   if (q.record_counter != nullptr && !q.counter_cleared) {
     const cudaError_t e = cudaMemsetAsync(q.record_counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
   }
-  if (lanes == 32) batch_query_start<32>(q, ir, ext, nlev, grid, block, smem, stream);
-  else if (lanes == 16) batch_query_start<16>(q, ir, ext, nlev, grid, block, smem, stream);
-  else if (lanes == 8) batch_query_start<8>(q, ir, ext, nlev, grid, block, smem, stream);
-  else batch_query_start<1>(q, ir, ext, nlev, grid, block, smem, stream);
+  if (lanes == 32) batch_query_start<32>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  else if (lanes == 16) batch_query_start<16>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  else if (lanes == 8) batch_query_start<8>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  else batch_query_start<1>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
   return cudaGetLastError();
 }
 
-cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, int grid,
-                         int block, cudaStream_t stream) {
-  if (q.num_lines <= 0 || q.n <= 0) return cudaSuccess;
-  if (block <= 0) block = 256;
-  if (block > 256) block = 256;
-  const int lanes =
-      lanes_per_record(uint64_t(q.num_lines), query_ir_descends(ir.bytes, q.ir_len));
+cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, cudaStream_t stream) {
+  if (q.num_lines <= 0 || q.n <= 0 || q.num_queries <= 0) return cudaSuccess;
+  constexpr int kBlock = 256;
+  QueryNeeds needs;
+  for (int i = 0; i < q.num_queries; ++i)
+    needs.add(ir.bytes + q.queries[i].ir_off, q.queries[i].ir_len);
+  // the queries of a launch are resident side by side
+  const uint64_t runs = uint64_t(q.num_lines) * uint64_t(q.num_queries);
+  const int lanes = lanes_per_record(runs, needs.descends);
   // partitions below 2 GiB take 32-bit positions whatever the result width
   // (700 MiB of posts, eight int64 slots: 427 us, 513 us before)
-  if (q.out64 == nullptr)
-    query_start_narrow(q, ir, q.out32, lanes, grid, block, stream);
+  if (!q.wide) query_start_narrow<int32_t>(q, ir, needs, lanes, runs, kBlock, stream);
   else if (q.n <= 0x7FFFFFFF)
-    query_start_narrow(q, ir, q.out64, lanes, grid, block, stream);
+    query_start_narrow<int64_t>(q, ir, needs, lanes, runs, kBlock, stream);
   else if (lanes == 32)
-    query_start<int64_t, int64_t, 32, 3>(q, ir, q.out64, grid, block, stream);
+    query_start<int64_t, int64_t, 32, 3>(q, ir, needs, kBlock, stream);
   else
-    query_start<int64_t, int64_t, 1, 3>(q, ir, q.out64, grid, block, stream);
+    query_start<int64_t, int64_t, 1, 3>(q, ir, needs, kBlock, stream);
   return cudaGetLastError();
 }
 

@@ -18,7 +18,17 @@ constexpr int kMaxQueryIrBytes = 4096;  // orig.hpp:11 kMaxQueryIrBytes
 // error bits (1, 2, 4), with which it shares the batch's error word.
 constexpr unsigned int kQueryStatusOverflow = 0x100u;
 
-// One query over every record of one partition.
+// Queries over every record of one partition, run by one launch (up to
+// kMaxLaunchQueries, their IR packed in the IrBlob).
+constexpr int kMaxLaunchQueries = 8;
+struct QueryOne {
+  int ir_off = 0;
+  int ir_len = 0;
+  int num_results = 0;           // result slots per record
+  int base_level = 0;            // bitmap level of query level 0 (1: elements
+                                 // of a top-level array are the records)
+  void *out = nullptr;           // [num_lines][num_results][2] int32 or int64
+};
 struct QueryLaunch {
   const uint8_t *in = nullptr;   // partition bytes
   int64_t n = 0;
@@ -27,13 +37,10 @@ struct QueryLaunch {
   const uint64_t *S = nullptr;   // string mask [W]
   const uint64_t *LB = nullptr;  // leveled bitmaps [L*W]
   int64_t W = 0;
-  int ir_len = 0;
-  int num_results = 0;           // result slots per record
   int num_levels = 0;            // levels present in LB; deeper reads see 0
-  int base_level = 0;            // bitmap level of query level 0 (1: elements
-                                 // of a top-level array are the records)
-  int32_t *out32 = nullptr;      // [num_lines][num_results][2], or
-  int64_t *out64 = nullptr;      // the same with 64-bit offsets
+  bool wide = false;             // 64-bit offsets in `out`
+  int num_queries = 1;
+  QueryOne queries[kMaxLaunchQueries];
   unsigned int *status = nullptr;  // kQueryStatusOverflow is OR-ed here (optional)
 };
 
@@ -43,8 +50,7 @@ struct IrBlob {
   uint8_t bytes[kMaxQueryIrBytes];
 };
 
-cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, int grid,
-                         int block, cudaStream_t stream);
+cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, cudaStream_t stream);
 
 // True when the IR holds extension opcodes (numeric filters, "..name", the
 // element checks of "[*]" and the open slices): those launch the

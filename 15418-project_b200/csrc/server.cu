@@ -567,17 +567,15 @@ struct gpj_server {
         ql.S = res->S;
         ql.LB = res->LB;
         ql.W = int64_t(res->W);
-        ql.ir_len = int(bq.ir_len);
-        ql.num_results = int(bq.num_result_slots);
         ql.num_levels = res->levels;
-        ql.base_level = int(bq.base_level);
-        ql.out32 = d_out + r->resp.result_offset[q];
+        ql.queries[0] = {0, int(bq.ir_len), int(bq.num_result_slots), int(bq.base_level),
+                         d_out + r->resp.result_offset[q]};
         ql.status = d_status;
         if (bq.num_result_slots == 0) continue;
         gpjb::IrBlob blob;
         std::memset(blob.bytes, 0, sizeof(blob.bytes));
         std::memcpy(blob.bytes, r->irs[q].data(), r->irs[q].size());
-        e = gpjb::query_launch(ql, blob, 0, 256, s.stream);
+        e = gpjb::query_launch(ql, blob, s.stream);
       }
       if (e == cudaSuccess)
         e = cudaMemcpyAsync(h_status, d_status, 4, cudaMemcpyDeviceToHost, s.stream);

@@ -158,3 +158,29 @@ def test_one_lane_at_every_block_count(cuda_ctx, gpj, blocks, query):
         np.testing.assert_array_equal(out.cpu().numpy().astype(np.int64), want)
     finally:
         cuda_ctx.free_index(ix)
+
+
+@pytest.mark.parametrize("kind", ["one", "eight", "nine", "long_ir"])
+@pytest.mark.parametrize("count", [60, 9000, 40000])
+def test_queries_of_one_host_call_share_launches(cuda_ctx, gpj, kind, count):
+    """gpj_query_host launches as many queries together as fit (8 queries, 4 KiB
+    of IR): plain, extension and descend queries side by side."""
+    data = np.frombuffer(_lines(5, count), np.uint8)
+    texts = {"one": QUERIES[:1], "eight": QUERIES[:8], "nine": QUERIES[4:13],
+             "long_ir": [("$.%s" % (ch * 1500), 0) for ch in "abcq"] + QUERIES[:2]}[kind]
+    comp = [gpj.compile(q, wildcard_limit=k) for q, k in texts]
+    levels = min(8, max(c.max_depth for c in comp))
+    host = torch.from_numpy(data.copy()).pin_memory()
+    outs = [torch.full((count, c.num_result_slots, 2), -7, dtype=torch.int32).pin_memory()
+            for c in comp]
+    try:
+        lines = cuda_ctx.query_host(host.data_ptr(), data.size, levels, comp,
+                                    [o.data_ptr() for o in outs], [o.numel() for o in outs])
+        assert lines == count
+    except gpj.CapacityError:  # raised after the copies: a slice was truncated
+        assert any(k for _, k in texts)
+    want_ix = oracle.OracleIndex(data, levels)
+    for c, o in zip(comp, outs):
+        np.testing.assert_array_equal(o.numpy().astype(np.int64),
+                                      want_ix.query(c.ir_bytes, c.num_result_slots),
+                                      err_msg=c.query_text)
