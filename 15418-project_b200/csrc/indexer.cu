@@ -281,16 +281,19 @@ __device__ __forceinline__ Agg tile_aggregate(uint32_t par, uint32_t dd, uint32_
 // tile by decoupled look-back while the compute warps run phase B of the
 // previous tile and phase A of the next.
 //
-// What bounds it is the integer work of the compute warps (about 1,380
+// What bounds it is the integer work of the compute warps (about 1,370
 // instructions per 4 KiB and warp) and how well the warps of an SM cover each
 // other's latencies and barriers.  One buffer per CTA (a tile's copy has phase
 // B of the previous tile to arrive) and 72 registers a thread (36 bytes
-// spilled) put three CTAs of 256 threads on an SM: 1 GiB of products 566 ->
+// spilled at first) put three CTAs of 256 threads on an SM: 1 GiB of products 566 ->
 // 528 us, of posts 591 -> 554 us against two CTAs with two buffers and 96
 // registers; three CTAs of 192 threads, with smaller tiles, were slower than
 // two of 256 (600 us).  Phase A has two barriers: a warp reads the escape carry
 // of its first row from the staged tile itself, and the decision to stop rides
-// on the first barrier (four barriers: 528 and 554 us, now 518 and 544).
+// on the first barrier (four barriers: 528 and 554 us, so 518 and 544).  Where
+// unstaged rows and the verify bitmaps lie is worked out on those paths only
+// (8 bytes spilled, 509 and 533 us), and quarters of at most one bracket store
+// into their slots without reading them (500 and 524 us).
 //
 // Claiming just in time keeps the time from a tile's claim to its aggregate
 // the same for every CTA (phase B of one tile plus phase A of the next), so
@@ -585,22 +588,20 @@ __device__ __forceinline__ bool phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
   uint32_t par0 = 0, thr_par = 0, par_ballot = 0, thr_nl = 0;
   int thr_d0 = 0, thr_t = 0;
   if (!stop) {
-    const IndexFile F = m.F;
-    const uint32_t ktile = m.tile - F.first_tile;
-    const uint64_t byte0 = uint64_t(ktile) * TILE_BYTES;
     const uint32_t valid = m.valid;
     const uint32_t row_byte = uint32_t(tid) * 128u;
-    const uint64_t lw0 = byte0 / 64u + 2u * uint64_t(tid);
     const bool row_in_smem = kTma && uint32_t(tid) < m.smem_rows;
     // rows past the end of the file read as zero bytes (no class)
     const uint32_t lim = valid > row_byte ? valid - row_byte : 0u;
-    const uint8_t *rp = P.in + F.in_off + byte0 + row_byte;
+    auto rp = [&] {
+      return P.in + m.F.in_off + uint64_t(m.tile - m.F.first_tile) * TILE_BYTES + row_byte;
+    };
     uint32_t r[16];
     if (row_in_smem) load_word_smem(sm.tile, tid, 0, r);
-    else load_word_global(rp, lim, 0, r);
+    else load_word_global(rp(), lim, 0, r);
     c0 = classify64(r);
     if (row_in_smem) load_word_smem(sm.tile, tid, 1, r);
-    else load_word_global(rp, lim, 64, r);
+    else load_word_global(rp(), lim, 64, r);
     c1 = classify64(r);
     const uint32_t tp0 = trailing_escape_parity(c0.bs);
     const uint32_t tp1 = trailing_escape_parity(c1.bs);
@@ -608,7 +609,7 @@ __device__ __forceinline__ bool phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
     if (lane == 0)
       cin0 = warp == 0
                  ? m.halo
-                 : escape_parity_before<kTma>(sm.tile, uint32_t(tid), m.smem_rows, rp, valid);
+                 : escape_parity_before<kTma>(sm.tile, uint32_t(tid), m.smem_rows, rp(), valid);
 
     const uint64_t E0 = escaped_bits(c0.bs, cin0);
     const uint64_t E1 = escaped_bits(c1.bs, tp0);
@@ -620,6 +621,8 @@ __device__ __forceinline__ bool phase_a(const IndexLaunch &P, PipeSmem<NT> &sm, 
     par0 = uint32_t(Sl0 >> 63);
     const uint32_t par1 = uint32_t(Sl1 >> 63);
     if (P.E != nullptr) {
+      const IndexFile F = m.F;
+      const uint64_t lw0 = uint64_t(m.tile - F.first_tile) * (NT * 2u) + 2u * uint64_t(tid);
       const uint64_t W = (F.n + 63u) / 64u;
       store2(P.E + F.s_off, lw0, W, E0 & valid_mask(lw0, F.n), E1 & valid_mask(lw0 + 1, F.n));
       store2(P.Q + F.s_off, lw0, W, Q0, Q1);
@@ -777,12 +780,15 @@ __device__ __forceinline__ void leveled_lane(LevelScratch<NT, LMAX, kList> &ls, 
       if (heavy) {
         items[listed + __popc(hb & lt)] = make_uint4(O, C, Pm, (d & 0xFFu) | (q << 8));
       } else {
-        // bit: the event, or 0 (below then covers the whole quarter)
+        // bit: the event, or 0 (below then covers the whole quarter).  Plain
+        // stores into cleared slots: an event leaves its level, and without
+        // one the second store replaces the first (both in the sink: neither
+        // is read)
         const uint32_t bit = ev & (0u - ev);
         const uint32_t below = bit - 1u;
-        wslot[min(d & 0xFFu, uint32_t(LMAX)) * 128 + q] |= (below & PO) | (bit & ~O);
-        const uint32_t d1 = d + ((O & bit) ? 1u : (bit ? 0xFFFFFFFFu : 0u));
-        wslot[min(d1 & 0xFFu, uint32_t(LMAX)) * 128 + q] |= PO & ~below;
+        const uint32_t d1 = d + uint32_t(__popc(O)) - uint32_t(__popc(C));
+        wslot[min(d1 & 0xFFu, uint32_t(LMAX)) * 128 + q] = PO & ~below;
+        wslot[min(d & 0xFFu, uint32_t(LMAX)) * 128 + q] = (below & PO) | (bit & ~O);
       }
       listed += __popc(hb);
       d += uint32_t(__popc(O)) - uint32_t(__popc(C));
