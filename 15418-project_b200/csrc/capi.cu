@@ -97,8 +97,14 @@ uint64_t round256(uint64_t x) { return (x + 255u) & ~uint64_t(255); }
 // is repeated with the exact size.
 uint64_t nl_capacity_guess(uint64_t n) { return n / 32u + 1024u; }
 
-// Sends the kernel's summary and error bits of a non-empty build straight to
-// the caller's four words (the error word is zeroed with the scratch).
+// The kernel can write a build's summary to the caller's words itself: there is
+// a kernel, and the words are aligned.
+bool summary_direct(uint64_t n, const uint64_t *d_summary) {
+  return n > 0 && d_summary != nullptr && (reinterpret_cast<uintptr_t>(d_summary) & 7u) == 0;
+}
+
+// Sends the kernel's summary and error bits straight to the caller's four words
+// (the error word is zeroed with the scratch).
 void bind_summary(gpjb::IndexLaunch &L, uint64_t *d_summary) {
   L.summary = reinterpret_cast<unsigned long long *>(d_summary);
   L.error = reinterpret_cast<unsigned int *>(d_summary + 3);
@@ -107,8 +113,8 @@ void bind_summary(gpjb::IndexLaunch &L, uint64_t *d_summary) {
 
 // Enqueues the fused indexer.  `in` may be unaligned: it is then copied into
 // the context's staging buffer first (TMA needs 16-byte aligned rows).  The
-// summary goes to d_summary where that is given and the input not empty, else
-// to the context's scratch.
+// summary goes to d_summary where summary_direct allows it, else to the
+// context's scratch.
 int enqueue_index(gpj_ctx *ctx, const uint8_t *in, uint64_t n, int levels,
                   uint32_t flags, const gpj_index &out, uint64_t *d_summary,
                   cudaStream_t stream) {
@@ -138,7 +144,7 @@ int enqueue_index(gpj_ctx *ctx, const uint8_t *in, uint64_t n, int levels,
   int rc = ensure(ctx->scratch, ctx->scratch_bytes, gpjb::index_scratch_bytes(n));
   if (rc != GPJ_OK) return rc;
   gpjb::index_bind_scratch(L, ctx->scratch);
-  if (n > 0 && d_summary != nullptr) bind_summary(L, d_summary);
+  if (summary_direct(n, d_summary)) bind_summary(L, d_summary);
 
   CUtensorMap map;
   bool tma = false;
@@ -650,11 +656,16 @@ int gpj_index_build_async(gpj_ctx *ctx, const uint8_t *d_input, uint64_t size_by
   index->num_levels = num_levels;
   rc = enqueue_index(ctx, d_input, size_bytes, num_levels, flags, *index, d_summary, stream);
   if (rc != GPJ_OK) return rc;
-  if (d_summary != nullptr && size_bytes == 0) {
-    GPJ_CUDA(cudaMemcpyAsync(d_summary, summary_ptr(ctx, size_bytes), 24,
-                             cudaMemcpyDeviceToDevice, stream),
+  if (d_summary != nullptr && !summary_direct(size_bytes, d_summary)) {
+    const unsigned long long *words = summary_ptr(ctx, size_bytes);
+    GPJ_CUDA(cudaMemcpyAsync(d_summary, words, 24, cudaMemcpyDeviceToDevice, stream),
              "copy summary");
-    GPJ_CUDA(cudaMemsetAsync(d_summary + 3, 0, 8, stream), "cudaMemsetAsync");
+    auto *error = reinterpret_cast<uint8_t *>(d_summary) + 24;
+    GPJ_CUDA(cudaMemsetAsync(error, 0, 8, stream), "cudaMemsetAsync");
+    if (size_bytes > 0)  // the word after the ticket counter
+      GPJ_CUDA(cudaMemcpyAsync(error, reinterpret_cast<const uint8_t *>(words) + 36, 4,
+                               cudaMemcpyDeviceToDevice, stream),
+               "copy error word");
   }
   return GPJ_OK;
 }

@@ -139,12 +139,24 @@ extern "C" int gpj_index_build_noalloc(const uint8_t *d_input, uint64_t size_byt
   bool tma = false;
   if ((flags & GPJ_INDEX_NO_TMA) == 0) tma = gpjb::index_make_tensor_map(&map, d_input, size_bytes);
 
-  // The kernel writes the summary and the error bits to the caller's words;
-  // index_launch clears the descriptors, counters and the error word before it.
-  L.summary = reinterpret_cast<unsigned long long *>(d_summary);
-  L.error = reinterpret_cast<unsigned int *>(d_summary + 3);
-  L.zero[0] = L.summary + 3;
-  const cudaError_t e = gpjb::index_launch(L, tma ? &map : nullptr, tma, stream);
+  // The kernel writes the summary and the error bits to the caller's words
+  // where they are aligned; index_launch clears the descriptors, counters and
+  // the error word before it.
+  const bool direct = (reinterpret_cast<uintptr_t>(d_summary) & 7u) == 0;
+  if (direct) {
+    L.summary = reinterpret_cast<unsigned long long *>(d_summary);
+    L.error = reinterpret_cast<unsigned int *>(d_summary + 3);
+    L.zero[0] = L.summary + 3;
+  }
+  cudaError_t e = gpjb::index_launch(L, tma ? &map : nullptr, tma, stream);
+  if (!direct) {
+    auto *error = reinterpret_cast<uint8_t *>(d_summary) + 24;
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(d_summary, L.summary, 24, cudaMemcpyDeviceToDevice, stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(error, 0, 8, stream);
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(error, L.error, 4, cudaMemcpyDeviceToDevice, stream);
+  }
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     return gpjb::report_error(GPJ_ERR_CUDA, cudaGetErrorString(e));

@@ -579,7 +579,7 @@ def run_ours(args, world, rank, local):
                 "h2d_bytes_per_step": sum(p1 - p0 for p0, p1 in parts),
                 "d2h_bytes_per_step": sum(h.numel() * 4 for hp in h_outs for h in hp),
                 "partitions": len(parts)},
-        "gpu_launches": 1 + len(comp),
+        "gpu_launches": 2 + len(comp),  # clear, index, queries
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
                      "kernel": "gpjb::index_kernel", "peak_kind": peak_kind,
@@ -834,7 +834,7 @@ def run_batch(args, world, rank, local):
         "e2e": {"value": round(gb / (e2e_ms / 1e3), 3), "unit": "GB/s",
                 "h2d_bytes_per_step": int(buf.size),
                 "d2h_bytes_per_step": int(v.result_ints) * 4 + v.num_files * 64},
-        "gpu_launches": 3,
+        "gpu_launches": 4,  # clear, index, finalize, query
         "roofline": {"bound": "hbm", "achieved": round(achieved, 1), "peak": peak,
                      "unit": "GB/s", "frac": round(achieved / peak, 4), "traffic": traffic,
                      "kernel": "gpjb::index_kernel (batched file table)", "peak_kind": peak_kind,
