@@ -1084,8 +1084,8 @@ __device__ uint32_t file_of_record(const BatchQueryLaunch &q, uint64_t r) {
   return lo;
 }
 
-template <bool kExt, int G>
-__global__ void __launch_bounds__(256, 4)
+template <bool kExt, int G, int kBlocks>
+__global__ void __launch_bounds__(256, kBlocks)
     batch_query_kernel(const BatchQueryLaunch q, const __grid_constant__ IrBlob ir, int nlev) {
   // every group's IR starts on a word and ends in kIrPad zero bytes
   __shared__ __align__(16) uint8_t s_ir[kMaxQueryIrBytes + kMaxBatchGroups * (kIrPad + 4)];
@@ -1337,14 +1337,14 @@ int lanes_per_record(uint64_t records, bool descends) {
   return 1;
 }
 
-template <int G>
+template <int G, int kBlocks>
 void batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, bool ext, int nlev, int grid,
                        int block, size_t smem, cudaStream_t stream) {
   // A plain launch: blocks that start beside the indexer's last CTAs keep the
   // SM split for those (200 KB of shared memory, little L1) for as long as they
   // run (1,500 MiB of files: 1,371 us a replay instead of 1,213).
-  if (ext) batch_query_kernel<true, G><<<grid, block, smem, stream>>>(q, ir, nlev);
-  else batch_query_kernel<false, G><<<grid, block, smem, stream>>>(q, ir, nlev);
+  if (ext) batch_query_kernel<true, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, nlev);
+  else batch_query_kernel<false, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, nlev);
 }
 
 // What the queries of a launch need together.
@@ -1425,10 +1425,25 @@ cudaError_t batch_query_launch(const BatchQueryLaunch &q, const IrBlob &ir, int 
     const cudaError_t e = cudaMemsetAsync(q.record_counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
   }
-  if (lanes == 32) batch_query_start<32>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-  else if (lanes == 16) batch_query_start<16>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-  else if (lanes == 8) batch_query_start<8>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-  else batch_query_start<1>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  if (lanes == 32) batch_query_start<32, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  if (lanes == 16) batch_query_start<16, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  if (lanes == 8) batch_query_start<8, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  if (lanes == 1) {
+    // Five blocks per SM where they hold all the records and four do not
+    // (157 K records: 125 us, 160 with four; 184 K: 134 and 170).  More records
+    // share out through the counter, and four are better (192 K: 155 us, 167
+    // with six; 216 K: 162 and 179; 588 K: 316 and 327 with five; 3.8 M: 1.62 ms
+    // and 1.94 with six).
+    const uint64_t one_each = resident_threads() / 4u;  // records of a block on every SM
+    const bool five = q.expected_records > 4u * one_each && q.expected_records <= 5u * one_each;
+    // Runs taken from the counter want no blocks beyond the resident ones: a
+    // later block's first run is its own and waits for it (192 K records: 169 us
+    // with eight blocks per SM in the grid, 155 with four; 274 K: 193 and 181).
+    if (q.record_counter != nullptr)
+      grid = int(std::min<uint64_t>(uint64_t(grid), one_each * (five ? 5u : 4u) / uint64_t(block)));
+    if (five) batch_query_start<1, 5>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+    else batch_query_start<1, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
+  }
   return cudaGetLastError();
 }
 

@@ -160,6 +160,36 @@ def test_one_lane_at_every_block_count(cuda_ctx, gpj, blocks, query):
         cuda_ctx.free_index(ix)
 
 
+@pytest.mark.parametrize("waves", [(4, 0), (4, 1), (5, 0), (5, 1), (9, 1)], ids=str)
+def test_one_lane_batch_at_every_block_count(gpj, waves):
+    """A batch's one-lane launches at both ends of the range that takes five
+    blocks per SM, and one whose warps take further runs of records."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    count = sms * 256 * waves[0] + waves[1]
+    part = _lines(78, 20000)
+    tail = b"\n".join(part.split(b"\n")[: count % 20000])
+    files = [part] * (count // 20000) + [tail]
+    c = gpj.compile("$.key.ab")
+    packed, offsets = gpj.pack_files(files)
+    dev = torch.from_numpy(packed).cuda()
+    table = [(o, len(f), 0) for o, f in zip(offsets, files)]
+    want = {f: oracle.OracleIndex(np.frombuffer(f, np.uint8), c.max_depth).query(
+        c.ir_bytes, c.num_result_slots) for f in (part, tail)}
+    with gpj.Batch(dev.data_ptr(), packed.size, table, [(c, 0, c.max_depth)]) as b:
+        for _ in range(2):
+            b.run()
+        torch.cuda.synchronize()
+        v = b.view()
+        from devmem import d2h
+        info = d2h(v.d_file_info, len(files) * 8, np.uint64).reshape(-1, 8)
+        got = d2h(v.d_results, v.result_ints, np.int32)
+        assert sum(int(row[0]) for row in info) == count
+        for f, row in zip(files, info):
+            lines, off = int(row[0]), int(row[3])
+            res = got[off:off + lines * c.num_result_slots * 2].reshape(lines, -1, 2)
+            np.testing.assert_array_equal(res.astype(np.int64), want[f])
+
+
 @pytest.mark.parametrize("kind", ["one", "eight", "nine", "long_ir"])
 @pytest.mark.parametrize("count", [60, 9000, 40000])
 def test_queries_of_one_host_call_share_launches(cuda_ctx, gpj, kind, count):
