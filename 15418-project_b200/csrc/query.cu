@@ -13,24 +13,6 @@
 namespace gpjb {
 namespace {
 
-enum : uint8_t {
-  OP_END = 0x00,
-  OP_STORE_RESULT = 0x01,
-  OP_MOVE_UP = 0x02,
-  OP_MOVE_DOWN = 0x03,
-  OP_MOVE_TO_KEY = 0x04,
-  OP_MOVE_TO_INDEX = 0x05,
-  OP_MOVE_TO_INDEX_REVERSE = 0x06,
-  OP_MARK_POSITION = 0x07,
-  OP_RESET_POSITION = 0x08,
-  OP_EXPRESSION_STRING_EQUALS = 0x09,
-  // Extensions of this build (never emitted for the reference's syntax):
-  OP_NUMBER_COMPARE = 0x0A,  // numeric filter: cmp byte, varint length, number text
-  OP_DESCEND_KEY = 0x0B,     // "..name" as the last step: varint length, key bytes
-  OP_EXPECT_AT_MOST = 0x0C,  // "[*]" element-count check: varint limit
-  OP_EXPECT_FOLLOWING = 0x0D,  // "[a:-b]": varint count of elements that must follow
-};
-
 constexpr unsigned kAll = 0xFFFFFFFFu;
 constexpr int kIrPad = 16;  // zero bytes after an IR in shared memory
 
@@ -265,23 +247,11 @@ __device__ __forceinline__ Pos prev_struct(const Rec<Pos> &c, const Group<G> &g,
   return found;
 }
 
-// query.cu:130-140 (LEB128).  Unsigned arithmetic reinterpreted as int, as
-// the reference's int result wraps; an operand longer than five bytes (never
-// produced by the compiler) reads as -1.
-__device__ __noinline__ int2 read_long_varint(const uint8_t *ir, int ir_len, int pos) {
-  uint32_t value = 0, byte = 0;
-  int shift = 0;
-  for (;;) {
-    byte = pos < ir_len ? ir[pos] : 0u;
-    ++pos;
-    if ((byte & 0x80u) == 0) break;
-    value |= (byte & 0x7Fu) << shift;
-    shift += 7;
-    if (shift > 28) return make_int2(-1, pos);
-  }
-  return make_int2(int(value | (byte << shift)), pos);
-}
 // The operand at pos; `first` is its first byte, nearly always the only one.
+__device__ __noinline__ int2 read_long_varint(const uint8_t *ir, int ir_len, int pos) {
+  const IrOperand o = ir_varint(ir, ir_len, pos);
+  return make_int2(o.value, o.next);
+}
 __device__ __forceinline__ int read_varint(const Query &q, int &pos, uint32_t first) {
   if (first < 0x80u) {
     ++pos;
@@ -826,8 +796,8 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
     case OP_MOVE_TO_KEY: {
       const int key_len = read_varint(q, qp, operand);
       const int key_pos = qp;
-      qp += key_len;
       if (key_len < 0 || !LEVEL_OK(level)) return;
+      qp = ir_skip(q.ir_len, qp, key_len);
       alive = alive && at(c, line_index) == '{';
       alive = find_key(c, q, g, alive, line_start, max_steps, ends[level * stride],
                        level_words(c, q.base + level), Key(q, key_pos, key_len), line_index, next,
@@ -937,8 +907,8 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
     case OP_EXPRESSION_STRING_EQUALS: {
       const int key_len = read_varint(q, qp, operand);
       const int key_pos = qp;
-      qp += key_len;
       if (key_len < 0 || !LEVEL_OK(level)) return;
+      qp = ir_skip(q.ir_len, qp, key_len);
       if (alive) {
         const Pos lend = ends[level * stride];
         while (at(c, line_index) == ' ' && line_index < lend) ++line_index;
@@ -956,8 +926,8 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       ++qp;
       const int lit_len = read_varint(q, qp, (window.x >> 16) & 0xFFu);
       const int lit_pos = qp;
+      if (lit_len < 0 || lit_len > q.ir_len - lit_pos || !LEVEL_OK(level)) return;
       qp += lit_len;
-      if (lit_len < 0 || lit_pos + lit_len > q.ir_len || !LEVEL_OK(level)) return;
       if (alive) {
         const Pos lend = ends[level * stride];
         while (at(c, line_index) == ' ' && line_index < lend) ++line_index;
@@ -983,8 +953,8 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       } else {
         const int key_len = read_varint(q, qp, operand);
         const int key_pos = qp;
-        qp += key_len;
         if (key_len < 0 || !LEVEL_OK(level)) return;
+        qp = ir_skip(q.ir_len, qp, key_len);
         if (alive)
           stored = descend(c, q, g, line_start, line_index, ends[level * stride], q.base + level,
                            Key(q, key_pos, key_len), stored, out, list, matches);
@@ -1192,7 +1162,7 @@ int query_ir_levels(const uint8_t *ir, int len) {
     case OP_MOVE_TO_KEY:
     case OP_EXPRESSION_STRING_EQUALS:
       skip_varint(p, &n);
-      if (n > 0) p += n;
+      if (n > 0) p = ir_skip(len, p, n);
       break;
     case OP_MOVE_TO_INDEX:
     case OP_MOVE_TO_INDEX_REVERSE:
@@ -1201,11 +1171,11 @@ int query_ir_levels(const uint8_t *ir, int len) {
     case OP_NUMBER_COMPARE:
       ++p;  // comparator
       skip_varint(p, &n);
-      if (n > 0) p += n;
+      if (n > 0) p = ir_skip(len, p, n);
       break;
     case OP_DESCEND_KEY:
       skip_varint(p, &n);
-      if (n > 0) p += n;
+      if (n > 0) p = ir_skip(len, p, n);
       break;
     case OP_MARK_POSITION:
       if (marked < kMaxQueryLevels) marks[marked++] = level;
@@ -1249,7 +1219,7 @@ bool query_ir_uses_extensions(const uint8_t *ir, int len) {
     case OP_MOVE_TO_KEY:
     case OP_EXPRESSION_STRING_EQUALS: {
       const int n = skip_varint(p);
-      if (n > 0) p += n;
+      if (n > 0) p = ir_skip(len, p, n);
       break;
     }
     case OP_MOVE_TO_INDEX:

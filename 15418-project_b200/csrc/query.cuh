@@ -5,11 +5,9 @@
 #include <cstdint>
 
 #include "indexer.cuh"
+#include "ir.cuh"
 
 namespace gpjb {
-
-constexpr int kMaxQueryLevels = 16;   // orig.hpp:10 kMaxQueryLevels
-constexpr int kMaxQueryIrBytes = 4096;  // orig.hpp:11 kMaxQueryIrBytes
 
 // Status bit a query raises when a record had more results than its slots:
 // a "[*]" array or open slice longer than the wildcard limit, or more
