@@ -67,4 +67,58 @@ __host__ __device__ __forceinline__ int ir_skip(int len, int pos, int bytes) {
   return bytes <= len - pos ? pos + bytes : len + 2;
 }
 
+// What running an IR takes.
+struct IrNeeds {
+  int levels = 1;         // query levels it can reach, at most kMaxQueryLevels
+  int marks = 0;          // marks open at once, at most kMaxQueryLevels
+  bool ext = false;       // it comes across an extension opcode
+  bool descends = false;  // it comes across DESCEND_KEY
+};
+
+// Follows the IR as the interpreter does (it has no jumps; reset returns to the
+// level of the last mark), up to where the interpreter leaves every record.
+inline IrNeeds ir_needs(const uint8_t *ir, int len) {
+  IrNeeds needs;
+  int level = 0, open = 0;
+  int marked[kMaxQueryLevels] = {};
+  for (int p = 0; p <= len + 1;) {
+    const uint8_t op = p < len ? ir[p] : uint8_t(OP_END);
+    ++p;
+    switch (op) {
+    case OP_END: return needs;
+    case OP_MOVE_UP: --level; break;
+    case OP_MOVE_DOWN:
+      ++level;
+      if (level + 1 > needs.levels && level < kMaxQueryLevels) needs.levels = level + 1;
+      break;
+    case OP_MARK_POSITION:
+      if (open == kMaxQueryLevels) return needs;
+      marked[open++] = level;
+      if (open > needs.marks) needs.marks = open;
+      break;
+    case OP_RESET_POSITION:
+      if (open == 0) return needs;
+      level = marked[--open];
+      break;
+    case OP_NUMBER_COMPARE: ++p; [[fallthrough]];  // comparator
+    case OP_DESCEND_KEY:
+    case OP_MOVE_TO_KEY:
+    case OP_EXPRESSION_STRING_EQUALS: {
+      if (op == OP_NUMBER_COMPARE || op == OP_DESCEND_KEY) needs.ext = true;
+      if (op == OP_DESCEND_KEY) needs.descends = true;
+      const IrOperand text = ir_varint(ir, len, p);
+      if (text.value < 0) return needs;
+      p = ir_skip(len, text.next, text.value);
+      break;
+    }
+    case OP_EXPECT_AT_MOST:
+    case OP_EXPECT_FOLLOWING: needs.ext = true; [[fallthrough]];
+    case OP_MOVE_TO_INDEX:
+    case OP_MOVE_TO_INDEX_REVERSE: p = ir_varint(ir, len, p).next; break;
+    default: break;
+    }
+  }
+  return needs;
+}
+
 }  // namespace gpjb

@@ -71,7 +71,7 @@ struct Query {
   int ir_len;
   int num_results;
   int base;  // bitmap level of query level 0
-  int nlev;  // levels the IR can reach (query_ir_levels)
+  int nlev, marks;  // levels and open marks there are slots for
 };
 
 // The reference reads file[] unguarded; well-formed JSON never leaves the
@@ -887,7 +887,7 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       break;
     }
     case OP_MARK_POSITION:
-      if (marked + 1 >= kMaxQueryLevels) return;
+      if (marked + 1 >= q.marks) return;
       ++marked;
       marks[marked * stride] = line_index;
       mark_levels[marked >> 3] &= ~(0xFFull << (8 * (marked & 7)));
@@ -1007,7 +1007,7 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
 template <typename Pos, typename OutT, bool kExt, int G, int kBlocks>
 __global__ void __launch_bounds__(256, kBlocks)
     query_kernel(const __grid_constant__ QueryLaunch q, const __grid_constant__ IrBlob ir,
-                 int nlev) {
+                 int nlev, int max_marks) {
   __shared__ __align__(16) uint8_t s_ir[kMaxQueryIrBytes + kIrPad];
   __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed<G>];
   __shared__ Pos s_match[kExt && G == 32 ? 8 : 1][32];
@@ -1018,7 +1018,7 @@ __global__ void __launch_bounds__(256, kBlocks)
   __syncthreads();
   const Group<G> g;
   const Rec<Pos> c{q.in, Pos(q.n), q.S, q.LB, Pos(q.W), q.num_levels, q.status};
-  const Query query{s_ir, one.ir_len, one.num_results, one.base_level, nlev};
+  const Query query{s_ir, one.ir_len, one.num_results, one.base_level, nlev, max_marks};
   OutT *const out = static_cast<OutT *>(one.out);
   Pos *ends = reinterpret_cast<Pos *>(s_state) + threadIdx.x;
   Pos *marks = ends + nlev * blockDim.x;
@@ -1056,7 +1056,8 @@ __device__ uint32_t file_of_record(const BatchQueryLaunch &q, uint64_t r) {
 
 template <bool kExt, int G, int kBlocks>
 __global__ void __launch_bounds__(256, kBlocks)
-    batch_query_kernel(const BatchQueryLaunch q, const __grid_constant__ IrBlob ir, int nlev) {
+    batch_query_kernel(const BatchQueryLaunch q, const __grid_constant__ IrBlob ir, int nlev,
+                       int max_marks) {
   // every group's IR starts on a word and ends in kIrPad zero bytes
   __shared__ __align__(16) uint8_t s_ir[kMaxQueryIrBytes + kMaxBatchGroups * (kIrPad + 4)];
   __shared__ int s_ir_off[kMaxBatchGroups];
@@ -1116,7 +1117,8 @@ __global__ void __launch_bounds__(256, kBlocks)
         const uint32_t now = __shfl_sync(kAll, qid, __ffs(int(left)) - 1);
         const bool mine = pending && qid == now;
         const BatchQueryGroup grp = q.groups[now];
-        const Query query{s_ir + s_ir_off[now], grp.ir_len, grp.num_results, grp.base_level, nlev};
+        const Query query{s_ir + s_ir_off[now], grp.ir_len, grp.num_results, grp.base_level, nlev,
+                          max_marks};
         run_records<int32_t, int32_t, kExt, G>(
             c, query, g, mine, start, end,
             q.out + row[kFiOutOff] + i * uint64_t(grp.num_results) * 2u, ends, marks,
@@ -1138,138 +1140,7 @@ __global__ void __launch_bounds__(256, kBlocks)
 
 }  // namespace
 
-int query_ir_levels(const uint8_t *ir, int len) {
-  // Follows the interpreter's level changes along the IR (it has no jumps;
-  // reset returns to a marked level) to find the deepest level it can reach.
-  int level = 0, deepest = 0, marked = 0;
-  int marks[kMaxQueryLevels] = {};
-  auto skip_varint = [&](int &p, int *value) {
-    uint32_t v = 0, b = 0;
-    int shift = 0;
-    while (p < len && ((b = ir[p++]) & 0x80u) != 0 && shift <= 28) {
-      v |= (b & 0x7Fu) << shift;
-      shift += 7;
-    }
-    if (value != nullptr) *value = int(v | (shift <= 28 ? (b << shift) : 0u));
-  };
-  for (int p = 0; p < len;) {
-    const uint8_t op = ir[p++];
-    if (op == OP_END) break;
-    int n = 0;
-    switch (op) {
-    case OP_MOVE_UP: --level; break;
-    case OP_MOVE_DOWN: ++level; break;
-    case OP_MOVE_TO_KEY:
-    case OP_EXPRESSION_STRING_EQUALS:
-      skip_varint(p, &n);
-      if (n > 0) p = ir_skip(len, p, n);
-      break;
-    case OP_MOVE_TO_INDEX:
-    case OP_MOVE_TO_INDEX_REVERSE:
-    case OP_EXPECT_AT_MOST:
-    case OP_EXPECT_FOLLOWING: skip_varint(p, nullptr); break;
-    case OP_NUMBER_COMPARE:
-      ++p;  // comparator
-      skip_varint(p, &n);
-      if (n > 0) p = ir_skip(len, p, n);
-      break;
-    case OP_DESCEND_KEY:
-      skip_varint(p, &n);
-      if (n > 0) p = ir_skip(len, p, n);
-      break;
-    case OP_MARK_POSITION:
-      if (marked < kMaxQueryLevels) marks[marked++] = level;
-      break;
-    case OP_RESET_POSITION:
-      if (marked > 0) level = marks[--marked];
-      break;
-    default: break;
-    }
-    if (level > deepest) deepest = level;
-  }
-  return deepest + 1 < kMaxQueryLevels ? deepest + 1 : kMaxQueryLevels;
-}
-
-// Mark slots an interpreter of the IR needs at most: its MARK_POSITION bytes
-// (a key's bytes may only add to them).
-int query_ir_marks(const uint8_t *ir, int len) {
-  int marks = 0;
-  for (int p = 0; p < len; ++p) marks += ir[p] == OP_MARK_POSITION ? 1 : 0;
-  return marks < kMaxQueryLevels ? marks : kMaxQueryLevels;
-}
-
-bool query_ir_uses_extensions(const uint8_t *ir, int len) {
-  auto skip_varint = [&](int &p) -> int {
-    uint32_t v = 0, b = 0;
-    int shift = 0;
-    while (p < len && ((b = ir[p++]) & 0x80u) != 0 && shift <= 28) {
-      v |= (b & 0x7Fu) << shift;
-      shift += 7;
-    }
-    return int(v | (shift <= 28 ? (b << shift) : 0u));
-  };
-  for (int p = 0; p < len;) {
-    const uint8_t op = ir[p++];
-    switch (op) {
-    case OP_END: return false;
-    case OP_NUMBER_COMPARE:
-    case OP_DESCEND_KEY:
-    case OP_EXPECT_AT_MOST:
-    case OP_EXPECT_FOLLOWING: return true;
-    case OP_MOVE_TO_KEY:
-    case OP_EXPRESSION_STRING_EQUALS: {
-      const int n = skip_varint(p);
-      if (n > 0) p = ir_skip(len, p, n);
-      break;
-    }
-    case OP_MOVE_TO_INDEX:
-    case OP_MOVE_TO_INDEX_REVERSE: skip_varint(p); break;
-    default: break;
-    }
-  }
-  return false;
-}
-
 namespace {
-
-// Does the interpreter come across DESCEND_KEY?  Follows the IR as the kernel
-// does (operands of up to five bytes, a fifth with the high bit reads as -1;
-// zero bytes past the end).
-bool query_ir_descends(const uint8_t *ir, int len) {
-  int p = 0;
-  auto byte_at = [&](int i) -> uint32_t { return i < len ? ir[i] : 0u; };
-  auto varint = [&]() -> int {
-    uint32_t v = 0, b = 0;
-    for (int shift = 0;;) {
-      b = byte_at(p++);
-      if ((b & 0x80u) == 0) return int(v | (b << shift));
-      v |= (b & 0x7Fu) << shift;
-      shift += 7;
-      if (shift > 28) return -1;
-    }
-  };
-  while (p <= len + 1) {
-    const uint32_t op = byte_at(p++);
-    switch (op) {
-    case OP_END: return false;
-    case OP_DESCEND_KEY: return true;
-    case OP_NUMBER_COMPARE: ++p; [[fallthrough]];
-    case OP_MOVE_TO_KEY:
-    case OP_EXPRESSION_STRING_EQUALS: {
-      const int n = varint();
-      if (n < 0 || n > len) return false;  // the kernel stops there too
-      p += n;
-      break;
-    }
-    case OP_MOVE_TO_INDEX:
-    case OP_MOVE_TO_INDEX_REVERSE:
-    case OP_EXPECT_AT_MOST:
-    case OP_EXPECT_FOLLOWING: varint(); break;
-    default: break;
-    }
-  }
-  return false;
-}
 
 uint64_t resident_threads() {
   static int sms_per_device[64] = {};
@@ -1307,40 +1178,58 @@ int lanes_per_record(uint64_t records, bool descends) {
   return 1;
 }
 
-template <int G, int kBlocks>
-void batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, bool ext, int nlev, int grid,
-                       int block, size_t smem, cudaStream_t stream) {
-  // A plain launch: blocks that start beside the indexer's last CTAs keep the
-  // SM split for those (200 KB of shared memory, little L1) for as long as they
-  // run (1,500 MiB of files: 1,371 us a replay instead of 1,213).
-  if (ext) batch_query_kernel<true, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, nlev);
-  else batch_query_kernel<false, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, nlev);
-}
-
 // What the queries of a launch need together.
-struct QueryNeeds {
-  int nlev = 1, marks = 0;
-  bool ext = false, descends = false;
+struct QueryNeeds : IrNeeds {
   void add(const uint8_t *ir, int len) {
-    nlev = std::max(nlev, query_ir_levels(ir, len));
-    marks = std::max(marks, query_ir_marks(ir, len));
-    ext = ext || query_ir_uses_extensions(ir, len);
-    descends = descends || query_ir_descends(ir, len);
+    const IrNeeds one = ir_needs(ir, len);
+    levels = std::max(levels, one.levels);
+    marks = std::max(marks, one.marks);
+    ext = ext || one.ext;
+    descends = descends || one.descends;
   }
 };
 
+// Dynamic shared memory of a block: a position per thread, level and mark.  Up
+// to 32 KiB fit beside a kernel's own arrays (10 KiB at most) in the 48 KiB a
+// launch may take unasked: all of 32-bit positions (256 threads, 16 levels, 16
+// marks), 64-bit ones up to 16 levels and marks together.
+template <typename Pos, typename Kernel>
+cudaError_t state_bytes(Kernel kernel, const QueryNeeds &needs, int block, size_t &bytes) {
+  bytes = size_t(needs.levels + needs.marks) * size_t(block) * sizeof(Pos);
+  if (bytes <= (32u << 10)) return cudaSuccess;
+  return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              int(2 * kMaxQueryLevels * 256 * sizeof(Pos)));
+}
+
+template <int G, int kBlocks>
+cudaError_t batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
+                              int grid, int block, cudaStream_t stream) {
+  // A plain launch: blocks that start beside the indexer's last CTAs keep the
+  // SM split for those (200 KB of shared memory, little L1) for as long as they
+  // run (1,500 MiB of files: 1,371 us a replay instead of 1,213).
+  auto kernel = needs.ext ? batch_query_kernel<true, G, kBlocks>
+                          : batch_query_kernel<false, G, kBlocks>;
+  size_t smem = 0;
+  const cudaError_t e = state_bytes<int32_t>(kernel, needs, block, smem);
+  if (e != cudaSuccess) return e;
+  kernel<<<grid, block, smem, stream>>>(q, ir, needs.levels, needs.marks);
+  return cudaGetLastError();
+}
+
 template <typename Pos, typename OutT, int G, int kBlocks>
-void query_start(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs, int block,
-                 cudaStream_t stream) {
+cudaError_t query_start(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs, int block,
+                        cudaStream_t stream) {
   const int64_t per_block = block / G;
   const dim3 grid(
       unsigned(std::min<int64_t>((q.num_lines + per_block - 1) / per_block, 0x7FFFFFFF)),
       unsigned(q.num_queries));
-  const size_t smem = size_t(needs.nlev + needs.marks) * size_t(block) * sizeof(Pos);
-  if (needs.ext)
-    query_kernel<Pos, OutT, true, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, needs.nlev);
-  else
-    query_kernel<Pos, OutT, false, G, kBlocks><<<grid, block, smem, stream>>>(q, ir, needs.nlev);
+  auto kernel = needs.ext ? query_kernel<Pos, OutT, true, G, kBlocks>
+                          : query_kernel<Pos, OutT, false, G, kBlocks>;
+  size_t smem = 0;
+  const cudaError_t e = state_bytes<Pos>(kernel, needs, block, smem);
+  if (e != cudaSuccess) return e;
+  kernel<<<grid, block, smem, stream>>>(q, ir, needs.levels, needs.marks);
+  return cudaGetLastError();
 }
 
 // Blocks per SM of the one-lane kernel.  Its blocks start together and take
@@ -1366,8 +1255,8 @@ int blocks_per_sm(uint64_t records) {
 }
 
 template <typename OutT>
-void query_start_narrow(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs, int lanes,
-                        uint64_t runs, int block, cudaStream_t stream) {
+cudaError_t query_start_narrow(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
+                               int lanes, uint64_t runs, int block, cudaStream_t stream) {
   if (lanes == 32) return query_start<int32_t, OutT, 32, 4>(q, ir, needs, block, stream);
   if (lanes == 16) return query_start<int32_t, OutT, 16, 4>(q, ir, needs, block, stream);
   if (lanes == 8) return query_start<int32_t, OutT, 8, 4>(q, ir, needs, block, stream);
@@ -1390,31 +1279,27 @@ cudaError_t batch_query_launch(const BatchQueryLaunch &q, const IrBlob &ir, int 
     const uint64_t blocks = (q.expected_records * uint64_t(lanes) + uint64_t(block) - 1) / block;
     grid = int(std::min<uint64_t>(uint64_t(grid), blocks));
   }
-  const size_t smem = size_t(needs.nlev + needs.marks) * size_t(block) * sizeof(int32_t);
   if (q.record_counter != nullptr && !q.counter_cleared) {
     const cudaError_t e = cudaMemsetAsync(q.record_counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
   }
-  if (lanes == 32) batch_query_start<32, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-  if (lanes == 16) batch_query_start<16, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-  if (lanes == 8) batch_query_start<8, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-  if (lanes == 1) {
-    // Five blocks per SM where they hold all the records and four do not
-    // (157 K records: 125 us, 160 with four; 184 K: 134 and 170).  More records
-    // share out through the counter, and four are better (192 K: 155 us, 167
-    // with six; 216 K: 162 and 179; 588 K: 316 and 327 with five; 3.8 M: 1.62 ms
-    // and 1.94 with six).
-    const uint64_t one_each = resident_threads() / 4u;  // records of a block on every SM
-    const bool five = q.expected_records > 4u * one_each && q.expected_records <= 5u * one_each;
-    // Runs taken from the counter want no blocks beyond the resident ones: a
-    // later block's first run is its own and waits for it (192 K records: 169 us
-    // with eight blocks per SM in the grid, 155 with four; 274 K: 193 and 181).
-    if (q.record_counter != nullptr)
-      grid = int(std::min<uint64_t>(uint64_t(grid), one_each * (five ? 5u : 4u) / uint64_t(block)));
-    if (five) batch_query_start<1, 5>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-    else batch_query_start<1, 4>(q, ir, needs.ext, needs.nlev, grid, block, smem, stream);
-  }
-  return cudaGetLastError();
+  if (lanes == 32) return batch_query_start<32, 4>(q, ir, needs, grid, block, stream);
+  if (lanes == 16) return batch_query_start<16, 4>(q, ir, needs, grid, block, stream);
+  if (lanes == 8) return batch_query_start<8, 4>(q, ir, needs, grid, block, stream);
+  // Five blocks per SM where they hold all the records and four do not
+  // (157 K records: 125 us, 160 with four; 184 K: 134 and 170).  More records
+  // share out through the counter, and four are better (192 K: 155 us, 167
+  // with six; 216 K: 162 and 179; 588 K: 316 and 327 with five; 3.8 M: 1.62 ms
+  // and 1.94 with six).
+  const uint64_t one_each = resident_threads() / 4u;  // records of a block on every SM
+  const bool five = q.expected_records > 4u * one_each && q.expected_records <= 5u * one_each;
+  // Runs taken from the counter want no blocks beyond the resident ones: a
+  // later block's first run is its own and waits for it (192 K records: 169 us
+  // with eight blocks per SM in the grid, 155 with four; 274 K: 193 and 181).
+  if (q.record_counter != nullptr)
+    grid = int(std::min<uint64_t>(uint64_t(grid), one_each * (five ? 5u : 4u) / uint64_t(block)));
+  return five ? batch_query_start<1, 5>(q, ir, needs, grid, block, stream)
+              : batch_query_start<1, 4>(q, ir, needs, grid, block, stream);
 }
 
 cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, cudaStream_t stream) {
@@ -1428,14 +1313,11 @@ cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, cudaStream_t st
   const int lanes = lanes_per_record(runs, needs.descends);
   // partitions below 2 GiB take 32-bit positions whatever the result width
   // (700 MiB of posts, eight int64 slots: 427 us, 513 us before)
-  if (!q.wide) query_start_narrow<int32_t>(q, ir, needs, lanes, runs, kBlock, stream);
-  else if (q.n <= 0x7FFFFFFF)
-    query_start_narrow<int64_t>(q, ir, needs, lanes, runs, kBlock, stream);
-  else if (lanes == 32)
-    query_start<int64_t, int64_t, 32, 3>(q, ir, needs, kBlock, stream);
-  else
-    query_start<int64_t, int64_t, 1, 3>(q, ir, needs, kBlock, stream);
-  return cudaGetLastError();
+  if (!q.wide) return query_start_narrow<int32_t>(q, ir, needs, lanes, runs, kBlock, stream);
+  if (q.n <= 0x7FFFFFFF)
+    return query_start_narrow<int64_t>(q, ir, needs, lanes, runs, kBlock, stream);
+  if (lanes == 32) return query_start<int64_t, int64_t, 32, 3>(q, ir, needs, kBlock, stream);
+  return query_start<int64_t, int64_t, 1, 3>(q, ir, needs, kBlock, stream);
 }
 
 }  // namespace gpjb

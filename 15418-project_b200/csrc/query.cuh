@@ -50,11 +50,6 @@ struct IrBlob {
 
 cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, cudaStream_t stream);
 
-// True when the IR holds extension opcodes (numeric filters, "..name", the
-// element checks of "[*]" and the open slices): those launch the
-// interpreter variant that has them.
-bool query_ir_uses_extensions(const uint8_t *ir, int len);
-
 // Batched query over every record of every file of a multi-file index build:
 // record r belongs to the file whose record range holds it (file_info from
 // index_finalize_files); the file's query group selects the IR (packed in the
