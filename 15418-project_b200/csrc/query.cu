@@ -9,6 +9,7 @@
 #include "query.cuh"
 
 #include <algorithm>
+#include <type_traits>
 
 namespace gpjb {
 namespace {
@@ -53,6 +54,10 @@ struct Group {
     return inc - v;
   }
 };
+
+// Counts the steps of a search loop.
+template <typename Pos>
+using Steps = std::make_unsigned_t<Pos>;
 
 template <typename Pos>
 struct Rec {
@@ -485,7 +490,7 @@ __device__ __forceinline__ void list_bits(uint16_t *list, uint64_t word, int fir
 // the others wait.
 template <typename Pos, int G>
 __device__ bool find_key(const Rec<Pos> &c, const Query &q, const Group<G> &g, bool active,
-                         Pos line_start, Pos max_steps, Pos level_end, const uint64_t *lvl,
+                         Pos line_start, Steps<Pos> max_steps, Pos level_end, const uint64_t *lvl,
                          const Key &key, Pos &line_index, Pos &next, uint16_t *list) {
   next = -1;
   bool found = false;
@@ -495,7 +500,7 @@ __device__ bool find_key(const Rec<Pos> &c, const Query &q, const Group<G> &g, b
   bool stray = active && lvl != nullptr && line_index < line_start;
   if (__any_sync(kAll, stray)) {
     if (stray) {
-      for (Pos steps = 1; steps <= max_steps; ++steps) {
+      for (Steps<Pos> steps = 1; steps <= max_steps; ++steps) {
         const Pos p1 = next_struct_lane(c, level_end, Pos(line_index + 1), lvl);
         line_index = p1;
         if (at(c, p1) != ':' ||
@@ -677,11 +682,11 @@ __device__ int descend(const Rec<Pos> &c, const Query &q, const Group<32> &g, Po
 // One lane.  Commas among the structural characters after line_index, up to
 // the first that is none or `limit` of them.
 template <typename Pos>
-__device__ int count_commas(const Rec<Pos> &c, Pos max_steps, Pos level_end, const uint64_t *lvl,
-                            Pos line_index, int limit) {
+__device__ int count_commas(const Rec<Pos> &c, Steps<Pos> max_steps, Pos level_end,
+                            const uint64_t *lvl, Pos line_index, int limit) {
   int commas = 0;
   Pos p = line_index;
-  for (Pos steps = 1; commas < limit && steps <= max_steps; ++steps) {
+  for (Steps<Pos> steps = 1; commas < limit && steps <= max_steps; ++steps) {
     p = next_struct_lane(c, level_end, Pos(p + 1), lvl);
     if (at(c, p) != ',') break;
     ++commas;
@@ -713,8 +718,8 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
     }
   }
   for (bool need = alive; __any_sync(kAll, need);) {
-    const Pos p = line_start + g.lane;
-    const unsigned hit = g.ballot(need && (p >= line_end || at(c, p) == '{'));
+    const bool past = line_end - line_start <= g.lane;
+    const unsigned hit = g.ballot(need && (past || at(c, Pos(line_start + g.lane)) == '{'));
     if (need) {
       line_start += hit != 0 ? __ffs(int(hit)) - 1 : G;
       need = hit == 0;
@@ -729,7 +734,8 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
   // new structural character of the record, so the bound is never reached;
   // on malformed input the reference's loops can revisit the same character
   // forever, and the record is abandoned instead.
-  const Pos max_steps = (line_end - line_start) + 2;
+  // (Unsigned: a record of 2^31 - 1 bytes has as many steps and two more.)
+  const Steps<Pos> max_steps = Steps<Pos>(line_end - line_start) + 2u;
   ends[0] = line_end;
   for (int i = 1; i < q.nlev; ++i) ends[i * stride] = -1;
   // A record still alive after an index step stands on that index, so the
@@ -784,8 +790,11 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       const bool fresh = alive && ends[level * stride] == -1;
       // right after a key search the end of the value is often known already
       const bool known = next_level == level - 1 && next > line_index;
-      Pos p = next_struct(c, g, fresh && !known, ends[(level - 1) * stride], Pos(line_index + 1),
-                          level_words(c, q.base + level - 1));
+      // (an empty object's key search ends one beyond its '}', and nothing
+      // follows that, nor might line_index + 1 be a position)
+      const Pos lend = ends[(level - 1) * stride];
+      Pos p = next_struct(c, g, fresh && !known && line_index < lend, lend,
+                          Pos(Steps<Pos>(line_index) + 1u), level_words(c, q.base + level - 1));
       if (known) p = next;
       if (fresh) {
         ends[level * stride] = p;
@@ -815,7 +824,7 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       int32_t ci = ch == '[' ? 0 : current + 1;
       const Pos lend = ends[level * stride];
       const uint64_t *lvl = level_words(c, q.base + level);
-      Pos steps = 0;
+      Steps<Pos> steps = 0;
       for (bool run = alive; __any_sync(kAll, run);) {
         bool forward = false, back = false;
         if (run) {
@@ -857,7 +866,7 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       alive = alive && (ch == ']' || ch == ',' || ch == '[');
       int32_t ci = ch == ']' ? 0 : current + 1;
       const uint64_t *lvl = level_words(c, q.base + level);
-      Pos steps = 0;
+      Steps<Pos> steps = 0;
       for (bool run = alive; __any_sync(kAll, run);) {
         bool forward = false, back = false;
         if (run) {
