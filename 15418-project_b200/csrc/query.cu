@@ -77,6 +77,7 @@ struct Query {
   int num_results;
   int base;  // bitmap level of query level 0
   int nlev, marks;  // levels and open marks there are slots for
+  bool ext;  // its own IR holds extension opcodes (others of the launch may, too)
 };
 
 // The reference reads file[] unguarded; well-formed JSON never leaves the
@@ -772,7 +773,8 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
           if ((2 * stored) % G == g.lane) out[2 * stored] = OutT(line_index);
           if ((2 * stored + 1) % G == g.lane) out[2 * stored + 1] = OutT(end_str);
         } else if constexpr (kExt) {
-          if (g.lane == 0) raise_status(c, kQueryStatusOverflow);  // only extension IR gets here
+          // (reference syntax may be given fewer slots than it stores)
+          if (q.ext && g.lane == 0) raise_status(c, kQueryStatusOverflow);
         }
       }
       ++stored;
@@ -1027,7 +1029,7 @@ __global__ void __launch_bounds__(256, kBlocks)
   __syncthreads();
   const Group<G> g;
   const Rec<Pos> c{q.in, Pos(q.n), q.S, q.LB, Pos(q.W), q.num_levels, q.status};
-  const Query query{s_ir, one.ir_len, one.num_results, one.base_level, nlev, max_marks};
+  const Query query{s_ir, one.ir_len, one.num_results, one.base_level, nlev, max_marks, one.ext};
   OutT *const out = static_cast<OutT *>(one.out);
   Pos *ends = reinterpret_cast<Pos *>(s_state) + threadIdx.x;
   Pos *marks = ends + nlev * blockDim.x;
@@ -1127,7 +1129,7 @@ __global__ void __launch_bounds__(256, kBlocks)
         const bool mine = pending && qid == now;
         const BatchQueryGroup grp = q.groups[now];
         const Query query{s_ir + s_ir_off[now], grp.ir_len, grp.num_results, grp.base_level, nlev,
-                          max_marks};
+                          max_marks, grp.ext};
         run_records<int32_t, int32_t, kExt, G>(
             c, query, g, mine, start, end,
             q.out + row[kFiOutOff] + i * uint64_t(grp.num_results) * 2u, ends, marks,
@@ -1189,12 +1191,13 @@ int lanes_per_record(uint64_t records, bool descends) {
 
 // What the queries of a launch need together.
 struct QueryNeeds : IrNeeds {
-  void add(const uint8_t *ir, int len) {
+  IrNeeds add(const uint8_t *ir, int len) {
     const IrNeeds one = ir_needs(ir, len);
     levels = std::max(levels, one.levels);
     marks = std::max(marks, one.marks);
     ext = ext || one.ext;
     descends = descends || one.descends;
+    return one;
   }
 };
 
@@ -1278,11 +1281,11 @@ cudaError_t query_start_narrow(const QueryLaunch &q, const IrBlob &ir, const Que
 
 }  // namespace
 
-cudaError_t batch_query_launch(const BatchQueryLaunch &q, const IrBlob &ir, int grid,
-                               int block, cudaStream_t stream) {
+cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,
+                               cudaStream_t stream) {
   QueryNeeds needs;
   for (int g = 0; g < q.num_groups; ++g)
-    needs.add(ir.bytes + q.groups[g].ir_off, q.groups[g].ir_len);
+    q.groups[g].ext = needs.add(ir.bytes + q.groups[g].ir_off, q.groups[g].ir_len).ext;
   const int lanes = lanes_per_record(q.expected_records, needs.descends);
   if (q.expected_records > 0) {
     const uint64_t blocks = (q.expected_records * uint64_t(lanes) + uint64_t(block) - 1) / block;
@@ -1311,12 +1314,12 @@ cudaError_t batch_query_launch(const BatchQueryLaunch &q, const IrBlob &ir, int 
               : batch_query_start<1, 4>(q, ir, needs, grid, block, stream);
 }
 
-cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, cudaStream_t stream) {
+cudaError_t query_launch(QueryLaunch q, const IrBlob &ir, cudaStream_t stream) {
   if (q.num_lines <= 0 || q.n <= 0 || q.num_queries <= 0) return cudaSuccess;
   constexpr int kBlock = 256;
   QueryNeeds needs;
   for (int i = 0; i < q.num_queries; ++i)
-    needs.add(ir.bytes + q.queries[i].ir_off, q.queries[i].ir_len);
+    q.queries[i].ext = needs.add(ir.bytes + q.queries[i].ir_off, q.queries[i].ir_len).ext;
   // the queries of a launch are resident side by side
   const uint64_t runs = uint64_t(q.num_lines) * uint64_t(q.num_queries);
   const int lanes = lanes_per_record(runs, needs.descends);

@@ -26,6 +26,7 @@ struct QueryOne {
   int base_level = 0;            // bitmap level of query level 0 (1: elements
                                  // of a top-level array are the records)
   void *out = nullptr;           // [num_lines][num_results][2] int32 or int64
+  bool ext = false;              // extension opcodes (query_launch sets it)
 };
 struct QueryLaunch {
   const uint8_t *in = nullptr;   // partition bytes
@@ -48,7 +49,7 @@ struct IrBlob {
   uint8_t bytes[kMaxQueryIrBytes];
 };
 
-cudaError_t query_launch(const QueryLaunch &q, const IrBlob &ir, cudaStream_t stream);
+cudaError_t query_launch(QueryLaunch q, const IrBlob &ir, cudaStream_t stream);
 
 // Batched query over every record of every file of a multi-file index build:
 // record r belongs to the file whose record range holds it (file_info from
@@ -61,6 +62,7 @@ struct BatchQueryGroup {
   int ir_len = 0;
   int num_results = 0;
   int base_level = 0;
+  bool ext = false;  // extension opcodes (batch_query_launch sets it)
 };
 struct BatchQueryLaunch {
   const uint8_t *in = nullptr;
@@ -86,7 +88,7 @@ struct BatchQueryLaunch {
   BatchQueryGroup groups[kMaxBatchGroups];
 };
 
-cudaError_t batch_query_launch(const BatchQueryLaunch &q, const IrBlob &ir, int grid,
-                               int block, cudaStream_t stream);
+cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,
+                               cudaStream_t stream);
 
 }  // namespace gpjb
