@@ -32,6 +32,7 @@ struct gpj_batch {
   std::vector<gpjb::IndexFile> files;
   std::vector<uint32_t> query_of_file;
   std::vector<gpjb::BatchQueryGroup> groups;
+  uint32_t used_groups = 0;  // bit g: some file names query g
   gpjb::IrBlob blob{};
   int max_levels = 0;
   // device state
@@ -137,6 +138,7 @@ gpjb::BatchQueryLaunch query_launch_of(const gpj_batch *b, bool after_index) {
   q.expected_records = b->records;
   q.num_groups = int(b->groups.size());
   for (size_t g = 0; g < b->groups.size(); ++g) q.groups[g] = b->groups[g];
+  q.used_groups = b->used_groups;
   return q;
 }
 
@@ -298,6 +300,7 @@ int gpj_batch_create(gpj_ctx *ctx, const uint8_t *d_input, uint64_t input_bytes,
     b->files[f].n = bf.size_bytes;
     b->files[f].levels = int32_t(queries[bf.query].num_levels);
     b->query_of_file[f] = bf.query;
+    b->used_groups |= 1u << bf.query;
     if (int(queries[bf.query].num_levels) > b->max_levels)
       b->max_levels = int(queries[bf.query].num_levels);
   }

@@ -1065,6 +1065,10 @@ __device__ uint32_t file_of_record(const BatchQueryLaunch &q, uint64_t r) {
   return lo;
 }
 
+__device__ __forceinline__ uint32_t group_of(const BatchQueryLaunch &q, const uint64_t *row) {
+  return row[kFiQuery] < uint64_t(q.num_groups) ? uint32_t(row[kFiQuery]) : 0u;
+}
+
 template <bool kExt, int G, int kBlocks>
 __global__ void __launch_bounds__(256, kBlocks)
     batch_query_kernel(const BatchQueryLaunch q, const __grid_constant__ IrBlob ir, int nlev,
@@ -1097,10 +1101,21 @@ __global__ void __launch_bounds__(256, kBlocks)
   const uint32_t chunk = uint32_t(share < kRecords ? kRecords : (share > 32u ? 32u : share));
   uint64_t base = (uint64_t(threadIdx.x / 32u) * gridDim.x + blockIdx.x) * chunk;
   while (base < records) {
+    const uint64_t end = base + chunk < records ? base + chunk : records;
     uint32_t f = file_of_record(q, base);
-    for (uint32_t k = 0; k < chunk && base + k < records; k += kRecords) {
-      const uint64_t r = base + k + uint32_t(g.shift / G);
-      bool pending = r < records;
+    for (uint64_t at = base; at < end; at += kRecords) {
+      if (q.group_mask != 0) {  // the same for the whole warp
+        for (f = __shfl_sync(kAll, f, 0); at < end; ++f) {
+          const uint64_t *row = q.file_info + uint64_t(f) * kFileInfoWords;
+          const uint64_t next = row[kFiRecOff] + row[kFiLines];
+          if (at >= next) continue;
+          if ((q.group_mask >> group_of(q, row)) & 1u) break;
+          at = next;
+        }
+        if (at >= end) break;
+      }
+      const uint64_t r = at + uint32_t(g.shift / G);
+      bool pending = r < end;
       uint64_t rec_off = 0, lines = 0;
       if (pending) {
         for (;; ++f) {  // the warp's later records may be in later files
@@ -1111,7 +1126,8 @@ __global__ void __launch_bounds__(256, kBlocks)
       }
       const uint64_t *row = q.file_info + uint64_t(f) * kFileInfoWords;
       const IndexFile F = q.files[f];
-      const uint32_t qid = row[kFiQuery] < uint64_t(q.num_groups) ? uint32_t(row[kFiQuery]) : 0u;
+      const uint32_t qid = group_of(q, row);
+      if (q.group_mask != 0) pending = pending && ((q.group_mask >> qid) & 1u) != 0;
       const uint64_t i = r - rec_off;
       const int64_t *nl = q.NL + row[kFiNlOff];
       // batch files are below 2 GiB (int32 results): 32-bit positions
@@ -1189,15 +1205,21 @@ int lanes_per_record(uint64_t records, bool descends) {
   return 1;
 }
 
+// Do queries with "..name" go in a launch of their own?  They make the launch a
+// warp per record for all its queries, which costs the others several times
+// their instructions where one lane each would do (2.3 M records of which one
+// small file asks "..id": query stage 5,696 us together, 1,318 apart).  Up to
+// there a launch of each after the other takes longer (1.5 K records: 35 and 54
+// us; 14 K runs in a host call: 290 and 327).
+bool descending_apart(uint64_t records) { return lanes_per_record(records, false) == 1; }
+
 // What the queries of a launch need together.
 struct QueryNeeds : IrNeeds {
-  IrNeeds add(const uint8_t *ir, int len) {
-    const IrNeeds one = ir_needs(ir, len);
+  void add(const IrNeeds &one) {
     levels = std::max(levels, one.levels);
     marks = std::max(marks, one.marks);
     ext = ext || one.ext;
     descends = descends || one.descends;
-    return one;
   }
 };
 
@@ -1279,13 +1301,8 @@ cudaError_t query_start_narrow(const QueryLaunch &q, const IrBlob &ir, const Que
   }
 }
 
-}  // namespace
-
-cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,
-                               cudaStream_t stream) {
-  QueryNeeds needs;
-  for (int g = 0; g < q.num_groups; ++g)
-    q.groups[g].ext = needs.add(ir.bytes + q.groups[g].ir_off, q.groups[g].ir_len).ext;
+cudaError_t batch_query_part(const BatchQueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
+                             int grid, int block, cudaStream_t stream) {
   const int lanes = lanes_per_record(q.expected_records, needs.descends);
   if (q.expected_records > 0) {
     const uint64_t blocks = (q.expected_records * uint64_t(lanes) + uint64_t(block) - 1) / block;
@@ -1314,12 +1331,9 @@ cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, i
               : batch_query_start<1, 4>(q, ir, needs, grid, block, stream);
 }
 
-cudaError_t query_launch(QueryLaunch q, const IrBlob &ir, cudaStream_t stream) {
-  if (q.num_lines <= 0 || q.n <= 0 || q.num_queries <= 0) return cudaSuccess;
+cudaError_t query_part(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
+                       cudaStream_t stream) {
   constexpr int kBlock = 256;
-  QueryNeeds needs;
-  for (int i = 0; i < q.num_queries; ++i)
-    q.queries[i].ext = needs.add(ir.bytes + q.queries[i].ir_off, q.queries[i].ir_len).ext;
   // the queries of a launch are resident side by side
   const uint64_t runs = uint64_t(q.num_lines) * uint64_t(q.num_queries);
   const int lanes = lanes_per_record(runs, needs.descends);
@@ -1330,6 +1344,55 @@ cudaError_t query_launch(QueryLaunch q, const IrBlob &ir, cudaStream_t stream) {
     return query_start_narrow<int64_t>(q, ir, needs, lanes, runs, kBlock, stream);
   if (lanes == 32) return query_start<int64_t, int64_t, 32, 3>(q, ir, needs, kBlock, stream);
   return query_start<int64_t, int64_t, 1, 3>(q, ir, needs, kBlock, stream);
+}
+
+}  // namespace
+
+cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,
+                               cudaStream_t stream) {
+  QueryNeeds needs[2];  // of the groups that do not descend, of those that do
+  uint32_t masks[2] = {0, 0};
+  for (int g = 0; g < q.num_groups; ++g) {
+    const IrNeeds one = ir_needs(ir.bytes + q.groups[g].ir_off, q.groups[g].ir_len);
+    q.groups[g].ext = one.ext;
+    if (((q.used_groups >> g) & 1u) == 0) continue;
+    needs[one.descends].add(one);
+    masks[one.descends] |= 1u << g;
+  }
+  const bool split = masks[0] != 0 && masks[1] != 0 && descending_apart(q.expected_records);
+  if (!split) {
+    needs[0].add(needs[1]);
+    return batch_query_part(q, ir, needs[0], grid, block, stream);
+  }
+  for (int d = 0; d < 2; ++d) {
+    q.group_mask = masks[d];
+    const cudaError_t e = batch_query_part(q, ir, needs[d], grid, block, stream);
+    if (e != cudaSuccess) return e;
+    q.counter_cleared = false;
+  }
+  return cudaSuccess;
+}
+
+cudaError_t query_launch(QueryLaunch q, const IrBlob &ir, cudaStream_t stream) {
+  if (q.num_lines <= 0 || q.n <= 0 || q.num_queries <= 0) return cudaSuccess;
+  QueryLaunch parts[2] = {q, q};  // the queries that do not descend, those that do
+  QueryNeeds needs[2];
+  parts[0].num_queries = parts[1].num_queries = 0;
+  for (int i = 0; i < q.num_queries; ++i) {
+    const IrNeeds one = ir_needs(ir.bytes + q.queries[i].ir_off, q.queries[i].ir_len);
+    q.queries[i].ext = one.ext;
+    QueryLaunch &part = parts[one.descends];
+    part.queries[part.num_queries++] = q.queries[i];
+    needs[one.descends].add(one);
+  }
+  const bool split = parts[0].num_queries > 0 && parts[1].num_queries > 0 &&
+                     descending_apart(uint64_t(q.num_lines) * uint64_t(q.num_queries));
+  if (!split) {
+    needs[0].add(needs[1]);
+    return query_part(q, ir, needs[0], stream);
+  }
+  const cudaError_t e = query_part(parts[0], ir, needs[0], stream);
+  return e != cudaSuccess ? e : query_part(parts[1], ir, needs[1], stream);
 }
 
 }  // namespace gpjb

@@ -49,6 +49,7 @@ struct IrBlob {
   uint8_t bytes[kMaxQueryIrBytes];
 };
 
+// One launch, or two where queries with "..name" (a warp per record) go apart.
 cudaError_t query_launch(QueryLaunch q, const IrBlob &ir, cudaStream_t stream);
 
 // Batched query over every record of every file of a multi-file index build:
@@ -86,8 +87,14 @@ struct BatchQueryLaunch {
   uint64_t expected_records = 0;
   int num_groups = 0;
   BatchQueryGroup groups[kMaxBatchGroups];
+  uint32_t used_groups = ~0u;  // bit g: some file is of group g
+  // groups whose files' records the launch runs, 0 for all of them
+  // (batch_query_launch sets it)
+  uint32_t group_mask = 0;
 };
 
+// One launch, or two where files with a "..name" query (a warp per record) go
+// apart: each passes over the other's files.
 cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,
                                cudaStream_t stream);
 
