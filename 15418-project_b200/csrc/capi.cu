@@ -84,6 +84,13 @@ int ensure(void *&buf, uint64_t &have, uint64_t need) {
   return GPJ_OK;
 }
 
+int ensure_copy_stream(gpj_ctx *ctx) {
+  if (ctx->copy_stream == nullptr)
+    GPJ_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking),
+             "cudaStreamCreate");
+  return GPJ_OK;
+}
+
 int bind_device(gpj_ctx *ctx) {
   if (ctx == nullptr) return fail(GPJ_ERR_INVALID_ARGUMENT, "null context");
   GPJ_CUDA(cudaSetDevice(ctx->device), "cudaSetDevice");
@@ -263,9 +270,8 @@ int enqueue_index_from_host(gpj_ctx *ctx, const uint8_t *h_in, uint8_t *d_in, ui
     if (rc != GPJ_OK) return rc;
     return enqueue_index(ctx, d_in, n, levels, 0u, out, nullptr, stream);
   }
-  if (ctx->copy_stream == nullptr)
-    GPJ_CUDA(cudaStreamCreateWithFlags(&ctx->copy_stream, cudaStreamNonBlocking),
-             "cudaStreamCreate");
+  int rc = ensure_copy_stream(ctx);
+  if (rc != GPJ_OK) return rc;
   if (ctx->piece_ready == nullptr)
     GPJ_CUDA(cudaEventCreateWithFlags(&ctx->piece_ready, cudaEventDisableTiming),
              "cudaEventCreate");
@@ -280,7 +286,7 @@ int enqueue_index_from_host(gpj_ctx *ctx, const uint8_t *h_in, uint8_t *d_in, ui
   L.NL = out.d_newline;
   L.nl_cap = out.newline_capacity;
   L.num_tiles = uint32_t(gpjb::index_num_tiles(n));
-  int rc = ensure(ctx->scratch, ctx->scratch_bytes, gpjb::index_scratch_bytes(n));
+  rc = ensure(ctx->scratch, ctx->scratch_bytes, gpjb::index_scratch_bytes(n));
   if (rc != GPJ_OK) return rc;
   gpjb::index_bind_scratch(L, ctx->scratch);
   CUtensorMap map;
@@ -329,6 +335,24 @@ int read_summary(gpj_ctx *ctx, uint64_t n, cudaStream_t stream, uint64_t *lines,
   *in_string = int(ctx->pinned[1]);
   *depth = int(int64_t(ctx->pinned[2]));
   return GPJ_OK;
+}
+
+// The scratch of gpj_results_compact.  A new one's header is cleared before
+// this returns and on a stream of the context's own: the caller's stream may be
+// capturing, and the clearing would then wait for the graph's first replay.
+int ensure_compact_scratch(gpj_ctx *ctx, uint64_t need) {
+  if (need <= ctx->compact_scratch_bytes && ctx->compact_scratch != nullptr) return GPJ_OK;
+  int rc = ensure_copy_stream(ctx);
+  if (rc == GPJ_OK) rc = ensure(ctx->compact_scratch, ctx->compact_scratch_bytes, need);
+  if (rc != GPJ_OK) return rc;
+  cudaError_t e =
+      cudaMemsetAsync(ctx->compact_scratch, 0, gpjb::kCompactHeaderBytes, ctx->copy_stream);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->copy_stream);
+  if (e == cudaSuccess) return GPJ_OK;
+  cudaFree(ctx->compact_scratch);
+  ctx->compact_scratch = nullptr;
+  ctx->compact_scratch_bytes = 0;
+  return cuda_fail(e, "clear compaction scratch");
 }
 
 constexpr size_t kSpareIndexBlocks = 4;
@@ -808,14 +832,8 @@ int gpj_results_compact(gpj_ctx *ctx, const int32_t *d_results, uint64_t num_lin
     return fail(GPJ_ERR_INVALID_ARGUMENT, "null match buffer");
   if (num_result_slots > 0 && num_lines > UINT64_MAX / num_result_slots / 2u)
     return fail(GPJ_ERR_OUT_OF_RANGE, "result array too large");
-  const uint64_t had = ctx->compact_scratch_bytes;
-  rc = ensure(ctx->compact_scratch, ctx->compact_scratch_bytes,
-              gpjb::compact_scratch_bytes(num_lines, num_result_slots));
+  rc = ensure_compact_scratch(ctx, gpjb::compact_scratch_bytes(num_lines, num_result_slots));
   if (rc != GPJ_OK) return rc;
-  if (ctx->compact_scratch_bytes != had)
-    GPJ_CUDA(cudaMemsetAsync(ctx->compact_scratch, 0, gpjb::kCompactHeaderBytes,
-                             static_cast<cudaStream_t>(stream_)),
-             "cudaMemsetAsync");
   GPJ_CUDA(gpjb::compact_launch(d_results, num_lines, num_result_slots, d_input, size_bytes,
                                 base_offset, d_matches, match_capacity, d_arena,
                                 arena_capacity,

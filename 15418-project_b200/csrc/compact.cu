@@ -119,7 +119,8 @@ __device__ __forceinline__ void block_scan(uint64_t &b, uint32_t &m, uint64_t &t
 }
 
 // `ticket` counts finished blocks (zero on entry; it wraps to zero with the
-// last one); the last block scans the counts of all writing blocks in place and writes the totals.
+// last one); the last block scans the counts of all writing blocks in place and
+// writes the totals.
 __global__ void __launch_bounds__(kCountThreads)
     count_kernel(const int32_t *res, uint64_t items, uint64_t n, BlockCounts *blocks,
                  uint32_t num_blocks, unsigned int *ticket, unsigned long long *counts) {
@@ -233,8 +234,8 @@ static_assert(sizeof(Record) == sizeof(gpj_match) && sizeof(Record) == 40, "five
 
 __global__ void __launch_bounds__(kThreads, 10)
     write_kernel(const int32_t *res, uint64_t items, uint32_t slots, const uint8_t *in, uint64_t n,
-                 int64_t base_offset, const BlockCounts *blocks, gpj_match *matches,
-                 uint64_t match_cap, uint8_t *arena, uint64_t arena_cap) {
+                 int64_t base_offset, const BlockCounts *blocks, unsigned int *ticket,
+                 gpj_match *matches, uint64_t match_cap, uint8_t *arena, uint64_t arena_cap) {
   __shared__ Record s_match[kItemsPerBlock];
   __shared__ uint32_t s_longer;  // bit 0: texts for a warp, bit 1: for the block
   const uint64_t first_item = uint64_t(blockIdx.x) * kItemsPerBlock;
@@ -252,6 +253,9 @@ __global__ void __launch_bounds__(kThreads, 10)
   block_scan<kThreads>(b, m, total_b, count);  // its barriers order s_longer as well
   // launched while the counting kernel runs; from here on its counts are there
   asm volatile("griddepcontrol.wait;" ::: "memory");
+  // The next call starts from zero whatever happened to the ticket: the last
+  // of several overlapping calls to get here follows all their counting.
+  if (blockIdx.x == 0 && threadIdx.x == 0) *ticket = 0;
   const BlockCounts before = blocks[blockIdx.x];
   // line and slot of the thread's first pair; the first line is the block's
   uint64_t line = first_item / slots;
@@ -379,8 +383,8 @@ cudaError_t compact_launch(const int32_t *d_results, uint64_t lines, uint32_t sl
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   return launch_overlapped(write_kernel, uint32_t(blocks), kThreads, 0, stream, d_results, items,
-                           slots, d_input, n, base_offset, bc, d_matches, match_cap, d_arena,
-                           arena_cap);
+                           slots, d_input, n, base_offset, bc, ticket, d_matches, match_cap,
+                           d_arena, arena_cap);
 }
 
 }  // namespace gpjb
