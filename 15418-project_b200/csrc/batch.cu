@@ -113,7 +113,7 @@ int bind_launch(gpj_batch *b) {
   L.NL = b->d_NL;
   L.nl_cap = b->d_NL ? b->nl_slots : 0;
   gpjb::index_bind_scratch(L, b->d_scratch);
-  L.zero[0] = reinterpret_cast<unsigned long long *>(b->d_totals + gpjb::kTotRecordCounter);
+  L.zero = reinterpret_cast<unsigned long long *>(b->d_totals + gpjb::kTotRecordCounter);
   b->tma = (b->flags & GPJ_INDEX_NO_TMA) == 0 &&
            gpjb::index_make_tensor_map(&b->map, b->d_input, b->input_bytes, b->index_threads);
   return GPJ_OK;

@@ -115,7 +115,7 @@ bool summary_direct(uint64_t n, const uint64_t *d_summary) {
 void bind_summary(gpjb::IndexLaunch &L, uint64_t *d_summary) {
   L.summary = reinterpret_cast<unsigned long long *>(d_summary);
   L.error = reinterpret_cast<unsigned int *>(d_summary + 3);
-  L.zero[0] = L.summary + 3;
+  L.zero = L.summary + 3;
 }
 
 // Enqueues the fused indexer.  `in` may be unaligned: it is then copied into

@@ -1117,18 +1117,14 @@ namespace {
 
 constexpr int kClearThreads = 256;
 
-// Zeroes the descriptors and counters, and up to two words elsewhere.
+// Zeroes the descriptors and counters, and a word elsewhere.
 __global__ void __launch_bounds__(kClearThreads)
-    clear_kernel(unsigned long long *words, uint64_t count, unsigned long long *a,
-                 unsigned long long *b) {
+    clear_kernel(unsigned long long *words, uint64_t count, unsigned long long *other) {
   asm volatile("griddepcontrol.launch_dependents;");
   const uint64_t stride = uint64_t(gridDim.x) * kClearThreads;
   for (uint64_t i = uint64_t(blockIdx.x) * kClearThreads + threadIdx.x; i < count; i += stride)
     words[i] = 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    if (a != nullptr) *a = 0;
-    if (b != nullptr) *b = 0;
-  }
+  if (blockIdx.x == 0 && threadIdx.x == 0 && other != nullptr) *other = 0;
 }
 
 cudaError_t launch_range(const IndexLaunch &L, const CUtensorMap *map, bool use_tma, bool overlap,
@@ -1148,7 +1144,7 @@ cudaError_t index_clear_scratch(const IndexLaunch &L, cudaStream_t stream) {
   const uint64_t words = uint64_t(L.num_tiles) + 8u;
   const uint64_t blocks = (words + kClearThreads - 1) / kClearThreads;
   clear_kernel<<<uint32_t(blocks < 148u ? blocks : 148u), kClearThreads, 0, stream>>>(
-      L.tile_state, words, L.zero[0], L.zero[1]);
+      L.tile_state, words, L.zero);
   return cudaGetLastError();
 }
 

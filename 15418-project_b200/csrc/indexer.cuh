@@ -52,8 +52,8 @@ struct IndexLaunch {
   unsigned int *tile_counter = nullptr;
   unsigned int *error = nullptr;
   unsigned long long *summary = nullptr;  // [0] lines [1] in-string [2] depth
-  // words outside the scratch that index_clear_scratch zeroes too (optional)
-  unsigned long long *zero[2] = {nullptr, nullptr};
+  // a word outside the scratch that index_clear_scratch zeroes too (optional)
+  unsigned long long *zero = nullptr;
   uint32_t num_tiles = 0;
   // tiles this launch claims: [tile_begin, tile_end); set by the launchers
   uint32_t tile_begin = 0, tile_end = 0;

@@ -146,7 +146,7 @@ extern "C" int gpj_index_build_noalloc(const uint8_t *d_input, uint64_t size_byt
   if (direct) {
     L.summary = reinterpret_cast<unsigned long long *>(d_summary);
     L.error = reinterpret_cast<unsigned int *>(d_summary + 3);
-    L.zero[0] = L.summary + 3;
+    L.zero = L.summary + 3;
   }
   cudaError_t e = gpjb::index_launch(L, tma ? &map : nullptr, tma, stream);
   if (!direct) {
