@@ -384,10 +384,15 @@ int gpj_batch_create(gpj_ctx *ctx, const uint8_t *d_input, uint64_t input_bytes,
     b->L.variant = best_v;
     best = 1e30f;
     int best_b = b->query_block, best_g = b->query_grid;
+    const gpjb::BatchQueryLaunch q = query_launch_of(b, true);
     for (int block : {128, 256}) {
+      int timed = 0;  // blocks of the last candidate: more may come to the same launch
       for (int gm : {4, 5, 8, 16}) {
         b->query_block = block;
         b->query_grid = sms * gm * (256 / block);
+        const int launched = gpjb::batch_query_grid(q, b->blob, b->query_grid, block);
+        if (launched == timed) continue;
+        timed = launched;
         const float ms = time_chain(b, s, 3);
         if (ms < best) {
           best = ms;
@@ -614,7 +619,8 @@ int gpj_batch_view_get(const gpj_batch *b, gpj_batch_view *v) {
   v->num_tiles = b->L.num_tiles;
   v->index_threads = uint32_t(b->index_threads);
   v->query_block = uint32_t(b->query_block);
-  v->query_grid = uint32_t(b->query_grid);
+  v->query_grid = uint32_t(gpjb::batch_query_grid(query_launch_of(b, true), b->blob, b->query_grid,
+                                                  b->query_block));
   v->uses_graph = b->exec != nullptr ? 1u : 0u;
   v->index_variant = b->L.variant;
   return GPJ_OK;

@@ -1301,34 +1301,47 @@ cudaError_t query_start_narrow(const QueryLaunch &q, const IrBlob &ir, const Que
   }
 }
 
-cudaError_t batch_query_part(const BatchQueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
-                             int grid, int block, cudaStream_t stream) {
-  const int lanes = lanes_per_record(q.expected_records, needs.descends);
+// Lanes per record, blocks and blocks per SM of a batch's query launch that may
+// take up to `grid` blocks.
+struct BatchShape {
+  int lanes, grid;
+  bool five = false;
+};
+BatchShape batch_shape(const BatchQueryLaunch &q, const QueryNeeds &needs, int grid, int block) {
+  BatchShape s{lanes_per_record(q.expected_records, needs.descends), grid};
   if (q.expected_records > 0) {
-    const uint64_t blocks = (q.expected_records * uint64_t(lanes) + uint64_t(block) - 1) / block;
-    grid = int(std::min<uint64_t>(uint64_t(grid), blocks));
+    const uint64_t blocks = (q.expected_records * uint64_t(s.lanes) + uint64_t(block) - 1) / block;
+    s.grid = int(std::min<uint64_t>(uint64_t(grid), blocks));
   }
-  if (q.record_counter != nullptr && !q.counter_cleared) {
-    const cudaError_t e = cudaMemsetAsync(q.record_counter, 0, sizeof(unsigned long long), stream);
-    if (e != cudaSuccess) return e;
-  }
-  if (lanes == 32) return batch_query_start<32, 4>(q, ir, needs, grid, block, stream);
-  if (lanes == 16) return batch_query_start<16, 4>(q, ir, needs, grid, block, stream);
-  if (lanes == 8) return batch_query_start<8, 4>(q, ir, needs, grid, block, stream);
+  if (s.lanes > 1) return s;
   // Five blocks per SM where they hold all the records and four do not
   // (157 K records: 125 us, 160 with four; 184 K: 134 and 170).  More records
   // share out through the counter, and four are better (192 K: 155 us, 167
   // with six; 216 K: 162 and 179; 588 K: 316 and 327 with five; 3.8 M: 1.62 ms
   // and 1.94 with six).
   const uint64_t one_each = resident_threads() / 4u;  // records of a block on every SM
-  const bool five = q.expected_records > 4u * one_each && q.expected_records <= 5u * one_each;
+  s.five = q.expected_records > 4u * one_each && q.expected_records <= 5u * one_each;
   // Runs taken from the counter want no blocks beyond the resident ones: a
   // later block's first run is its own and waits for it (192 K records: 169 us
   // with eight blocks per SM in the grid, 155 with four; 274 K: 193 and 181).
   if (q.record_counter != nullptr)
-    grid = int(std::min<uint64_t>(uint64_t(grid), one_each * (five ? 5u : 4u) / uint64_t(block)));
-  return five ? batch_query_start<1, 5>(q, ir, needs, grid, block, stream)
-              : batch_query_start<1, 4>(q, ir, needs, grid, block, stream);
+    s.grid = int(std::min<uint64_t>(uint64_t(s.grid),
+                                    one_each * (s.five ? 5u : 4u) / uint64_t(block)));
+  return s;
+}
+
+cudaError_t batch_query_part(const BatchQueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
+                             int grid, int block, cudaStream_t stream) {
+  const BatchShape s = batch_shape(q, needs, grid, block);
+  if (q.record_counter != nullptr && !q.counter_cleared) {
+    const cudaError_t e = cudaMemsetAsync(q.record_counter, 0, sizeof(unsigned long long), stream);
+    if (e != cudaSuccess) return e;
+  }
+  if (s.lanes == 32) return batch_query_start<32, 4>(q, ir, needs, s.grid, block, stream);
+  if (s.lanes == 16) return batch_query_start<16, 4>(q, ir, needs, s.grid, block, stream);
+  if (s.lanes == 8) return batch_query_start<8, 4>(q, ir, needs, s.grid, block, stream);
+  return s.five ? batch_query_start<1, 5>(q, ir, needs, s.grid, block, stream)
+                : batch_query_start<1, 4>(q, ir, needs, s.grid, block, stream);
 }
 
 cudaError_t query_part(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
@@ -1346,27 +1359,40 @@ cudaError_t query_part(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds 
   return query_start<int64_t, int64_t, 1, 3>(q, ir, needs, kBlock, stream);
 }
 
+// A batch's groups by launch: those that do not descend and those that do where
+// they go apart (`split`), else all of them in the first.  Marks the groups with
+// extension opcodes.
+struct BatchParts {
+  QueryNeeds needs[2];
+  uint32_t masks[2] = {0, 0};
+  bool split;
+  BatchParts(BatchQueryLaunch &q, const IrBlob &ir) {
+    for (int g = 0; g < q.num_groups; ++g) {
+      const IrNeeds one = ir_needs(ir.bytes + q.groups[g].ir_off, q.groups[g].ir_len);
+      q.groups[g].ext = one.ext;
+      if (((q.used_groups >> g) & 1u) == 0) continue;
+      needs[one.descends].add(one);
+      masks[one.descends] |= 1u << g;
+    }
+    split = masks[0] != 0 && masks[1] != 0 && descending_apart(q.expected_records);
+    if (!split) needs[0].add(needs[1]);
+  }
+};
+
 }  // namespace
+
+int batch_query_grid(BatchQueryLaunch q, const IrBlob &ir, int grid, int block) {
+  const BatchParts parts(q, ir);
+  return batch_shape(q, parts.needs[0], grid, block).grid;
+}
 
 cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,
                                cudaStream_t stream) {
-  QueryNeeds needs[2];  // of the groups that do not descend, of those that do
-  uint32_t masks[2] = {0, 0};
-  for (int g = 0; g < q.num_groups; ++g) {
-    const IrNeeds one = ir_needs(ir.bytes + q.groups[g].ir_off, q.groups[g].ir_len);
-    q.groups[g].ext = one.ext;
-    if (((q.used_groups >> g) & 1u) == 0) continue;
-    needs[one.descends].add(one);
-    masks[one.descends] |= 1u << g;
-  }
-  const bool split = masks[0] != 0 && masks[1] != 0 && descending_apart(q.expected_records);
-  if (!split) {
-    needs[0].add(needs[1]);
-    return batch_query_part(q, ir, needs[0], grid, block, stream);
-  }
+  const BatchParts parts(q, ir);
+  if (!parts.split) return batch_query_part(q, ir, parts.needs[0], grid, block, stream);
   for (int d = 0; d < 2; ++d) {
-    q.group_mask = masks[d];
-    const cudaError_t e = batch_query_part(q, ir, needs[d], grid, block, stream);
+    q.group_mask = parts.masks[d];
+    const cudaError_t e = batch_query_part(q, ir, parts.needs[d], grid, block, stream);
     if (e != cudaSuccess) return e;
     q.counter_cleared = false;
   }

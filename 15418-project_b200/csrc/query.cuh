@@ -93,6 +93,10 @@ struct BatchQueryLaunch {
   uint32_t group_mask = 0;
 };
 
+// Blocks that batch_query_launch starts of the `grid` it may (in its first launch
+// where it makes two).
+int batch_query_grid(BatchQueryLaunch q, const IrBlob &ir, int grid, int block);
+
 // One launch, or two where files with a "..name" query (a warp per record) go
 // apart: each passes over the other's files.
 cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,

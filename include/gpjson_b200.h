@@ -326,7 +326,7 @@ typedef struct gpj_batch_view {
   uint32_t num_tiles;
   uint32_t index_threads; /* indexer CTA size: tiles of index_threads * 128 B */
   uint32_t query_block;
-  uint32_t query_grid;
+  uint32_t query_grid;    /* blocks the query launch starts */
   uint32_t uses_graph;
   uint32_t index_variant; /* indexer variant bits for up to 4 levels: 1 = each lane walks its
                              own leveled quarters (no per-warp list), 2 = look-back rounds of
