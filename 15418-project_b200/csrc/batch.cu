@@ -526,7 +526,7 @@ int run_in_pieces(gpj_batch *b, const uint8_t *h_input, cudaStream_t stream) {
     BCUDA(cudaEventCreateWithFlags(&b->piece_ready, cudaEventDisableTiming), "cudaEventCreate");
   auto *d_in = const_cast<uint8_t *>(b->d_input);
   const CUtensorMap *map = b->tma ? &b->map : nullptr;
-  BCUDA(gpjb::index_clear_scratch(b->L, stream), "cudaMemsetAsync");
+  BCUDA(gpjb::index_clear_scratch(b->L, stream), "index scratch clearing launch");
   // the copies start after the work already queued on `stream`
   BCUDA(cudaEventRecord(b->piece_ready, stream), "cudaEventRecord");
   BCUDA(cudaStreamWaitEvent(b->copy_stream, b->piece_ready, 0), "cudaStreamWaitEvent");

@@ -173,7 +173,7 @@ int enqueue_index(gpj_ctx *ctx, const uint8_t *in, uint64_t n, int levels,
       return fail(GPJ_ERR_INVALID_ARGUMENT,
                   "GPJ_INDEX_DIAG_TILE0_UNPUBLISHED needs an input of at least two tiles");
     L.lookback_spin_limit = 1u << 14;
-    GPJ_CUDA(gpjb::index_clear_scratch(L, stream), "cudaMemsetAsync");
+    GPJ_CUDA(gpjb::index_clear_scratch(L, stream), "index scratch clearing launch");
     GPJ_CUDA(gpjb::index_launch_range(L, tma ? &map : nullptr, tma, stream, 1u, L.num_tiles),
              "index kernel launch");
     return GPJ_OK;
@@ -291,7 +291,7 @@ int enqueue_index_from_host(gpj_ctx *ctx, const uint8_t *h_in, uint8_t *d_in, ui
   gpjb::index_bind_scratch(L, ctx->scratch);
   CUtensorMap map;
   const bool tma = gpjb::index_make_tensor_map(&map, d_in, n);
-  GPJ_CUDA(gpjb::index_clear_scratch(L, stream), "cudaMemsetAsync");
+  GPJ_CUDA(gpjb::index_clear_scratch(L, stream), "index scratch clearing launch");
   // the copies start after the work already queued on `stream`
   GPJ_CUDA(cudaEventRecord(ctx->piece_ready, stream), "cudaEventRecord");
   GPJ_CUDA(cudaStreamWaitEvent(ctx->copy_stream, ctx->piece_ready, 0), "cudaStreamWaitEvent");

@@ -26,7 +26,9 @@ bool host_range_mapped(const void *p, uint64_t bytes);
 // Up to this size a host input is read by copy_many instead of the copy
 // engine: a copy of its own takes the engine 5-6 us beside the bytes' time at
 // 55 GB/s, a kernel reads them together (21 files, 4 MiB in all: 80 us for 190;
-// a burst of 40 requests 1,414 -> 1,171 us with the results moved likewise).
+// a burst of 40 requests 1,414 -> 1,171 us with the results moved likewise; a
+// burst from buffers never read before 1,320 us, 1,515 with the engine for the
+// inputs).
 constexpr uint64_t kCopyManyMaxInput = 1u << 20;
 // The same for results, which are mostly a few KiB.
 constexpr uint64_t kCopyManyMaxResult = 256u << 10;

@@ -284,16 +284,15 @@ __device__ __forceinline__ Agg tile_aggregate(uint32_t par, uint32_t dd, uint32_
 // What bounds it is the integer work of the compute warps (about 1,370
 // instructions per 4 KiB and warp) and how well the warps of an SM cover each
 // other's latencies and barriers.  One buffer per CTA (a tile's copy has phase
-// B of the previous tile to arrive) and 72 registers a thread (36 bytes
-// spilled at first) put three CTAs of 256 threads on an SM: 1 GiB of products 566 ->
-// 528 us, of posts 591 -> 554 us against two CTAs with two buffers and 96
-// registers; three CTAs of 192 threads, with smaller tiles, were slower than
-// two of 256 (600 us).  Phase A has two barriers: a warp reads the escape carry
-// of its first row from the staged tile itself, and the decision to stop rides
-// on the first barrier (four barriers: 528 and 554 us, so 518 and 544).  Where
-// unstaged rows and the verify bitmaps lie is worked out on those paths only
-// (8 bytes spilled, 509 and 533 us), and quarters of at most one bracket store
-// into their slots without reading them (500 and 524 us).
+// B of the previous tile to arrive) and 72 registers a thread put three CTAs of
+// 256 threads on an SM: 1 GiB of products 528 us, 566 with two CTAs of two
+// buffers and 96 registers; 600 with three CTAs of 192 threads, whose tiles are
+// smaller.  Phase A has two barriers (a warp reads the escape carry of its first
+// row from the staged tile itself, the decision to stop rides on the first
+// barrier): 518 us, 528 with four.  To live with 72 registers, where unstaged
+// rows and the verify bitmaps lie is worked out on those paths only (509 us),
+// and quarters of at most one bracket store into their slots without reading
+// them (500 us).
 //
 // Claiming just in time keeps the time from a tile's claim to its aggregate
 // the same for every CTA (phase B of one tile plus phase A of the next), so

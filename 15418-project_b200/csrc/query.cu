@@ -1185,17 +1185,20 @@ uint64_t resident_threads() {
 
 // Lanes per record.  More lanes shorten a record's chain of dependent loads
 // and instructions but execute more instructions per record in total (a
-// round of the group's search costs about the same for 8 lanes as for 32), so
-// the most lanes win as long as all records are resident at once (four
-// 256-thread blocks per SM) and one lane wins beyond.  Measured for
-// $.user.lang on post records (us, one / 8 / 16 / 32 lanes, before this
-// split): 437 records 38 / 20.5 / 14 / 11 (53), 3.5 K 40 / 22.6 / 16.4 / 12.9
-// (55), 7 K 39.4 / 23.1 / 17.4 / 20.6 (56), 14 K 41 / 24.6 / 26 / 33 (55),
-// 28 K 50 / 44 / 48 / 66 (67), 56 K 67 / 75 / 90 / 125 (85); with more opcodes
-// (eight-slot arrays) 14 K records 90 / 83 / 127 / 163 (110), 28 K 115 / 165 /
-// 218 / 293 (140).  "..name" reads every level's words of the whole record,
-// which only a wide group reads in whole sectors: 41 K records 897 us with one
-// lane, 293 with 8, 231 with 32 (200 with the search of descend).
+// round of the group's search costs about the same for 8 lanes as for 32).
+// The launch takes the most lanes with which all records are resident at once
+// (four 256-thread blocks per SM), and one lane beyond.  Measured (us, one / 8
+// / 16 / 32 lanes, one thread per record before this split in brackets) for
+// $.user.lang on posts: 437 records 38 / 20.5 / 14 / 11 (53), 3.5 K 40 / 22.6 /
+// 16.4 / 12.9 (55), 7 K 39.4 / 23.1 / 17.4 / 20.6 (56), 14 K 41 / 24.6 / 26 / 33
+// (55), 28 K 50 / 44 / 48 / 66 (67), 56 K 67 / 75 / 90 / 125 (85); for
+// eight-slot arrays 14 K records 90 / 83 / 127 / 163 (110), 28 K 115 / 165 / 218
+// / 293 (140).  Where one lane begins to win depends on the IR, at which the
+// rule does not look: its line (19 K records) lies between the short IR's, which
+// loses 6 us at 28 K by it, and the eight-slot one's, which gains 50 there.
+// "..name" reads every level's words of the whole record, which only a wide
+// group reads in whole sectors: 41 K records 897 us with one lane of this
+// kernel, 293 with 8, 231 with 32 (200 with the search of descend).
 int lanes_per_record(uint64_t records, bool descends) {
   if (descends) return 32;
   if (records == 0) return 1;
@@ -1268,11 +1271,13 @@ cudaError_t query_start(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds
 
 // Blocks per SM of the one-lane kernel.  Its blocks start together and take
 // about as long as each other, so a launch runs in waves, and a wave takes time
-// in proportion to the blocks of it per SM from four on ($.user.lang on posts:
-// 76, 98 and 126 us for a full wave of four, five and six): the fewest waves
+// about in proportion to the blocks of it per SM from four on: the fewest waves
 // times blocks win, fewer blocks where two are equal.  153 K array elements:
 // 87, 71 and 78 us with four, five and six; 208 K: 111, 124 and 102; 236 K:
-// 113, 128 and 160; 349 K: 165, 145 and 182.
+// 113, 128 and 160; 349 K: 165, 145 and 182.  (Full waves of $.user.lang on
+// posts take 76, 98 and 126 us, a little more than 4 : 5 : 6.  By those weights
+// 606 to 682 K records would take four blocks instead of six, which array
+// elements want, 265 us for 290, and posts do not, 366 for 338.)
 int blocks_per_sm(uint64_t records) {
   const uint64_t per_block = resident_threads() / 4u;  // one block on every SM
   int best = 4;
