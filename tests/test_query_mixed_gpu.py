@@ -5,6 +5,7 @@ import pytest
 import torch
 
 import oracle
+from kernel_trace import launches
 
 pytestmark = pytest.mark.gpu
 
@@ -76,12 +77,7 @@ def test_an_extension_query_beside_a_plain_one_keeps_its_status(cuda_ctx, gpj):
 
 
 def _query_kernels(run):
-    run()
-    torch.cuda.synchronize()
-    with torch.profiler.profile(activities=[torch.profiler.ProfilerActivity.CUDA]) as prof:
-        run()
-        torch.cuda.synchronize()
-    return {e.name for e in prof.events() if "query_kernel" in e.name}
+    return {name for name, _, _ in launches(run, "query_kernel")}
 
 
 def test_a_descending_query_leaves_the_others_their_kernels(cuda_ctx, gpj):
