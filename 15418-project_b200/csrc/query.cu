@@ -1069,7 +1069,8 @@ __device__ __forceinline__ uint32_t group_of(const BatchQueryLaunch &q, const ui
   return row[kFiQuery] < uint64_t(q.num_groups) ? uint32_t(row[kFiQuery]) : 0u;
 }
 
-template <bool kExt, int G, int kBlocks>
+// kPart: the launch runs the records of some groups' files only (group_mask).
+template <bool kExt, int G, int kBlocks, bool kPart>
 __global__ void __launch_bounds__(256, kBlocks)
     batch_query_kernel(const BatchQueryLaunch q, const __grid_constant__ IrBlob ir, int nlev,
                        int max_marks) {
@@ -1101,10 +1102,11 @@ __global__ void __launch_bounds__(256, kBlocks)
   const uint32_t chunk = uint32_t(share < kRecords ? kRecords : (share > 32u ? 32u : share));
   uint64_t base = (uint64_t(threadIdx.x / 32u) * gridDim.x + blockIdx.x) * chunk;
   while (base < records) {
-    const uint64_t end = base + chunk < records ? base + chunk : records;
     uint32_t f = file_of_record(q, base);
-    for (uint64_t at = base; at < end; at += kRecords) {
-      if (q.group_mask != 0) {  // the same for the whole warp
+    for (uint32_t k = 0; k < chunk && base + k < records; k += kRecords) {
+      if constexpr (kPart) {  // to the next record of the launch's groups, if the run has one
+        const uint64_t end = base + chunk < records ? base + chunk : records;
+        uint64_t at = base + k;
         for (f = __shfl_sync(kAll, f, 0); at < end; ++f) {
           const uint64_t *row = q.file_info + uint64_t(f) * kFileInfoWords;
           const uint64_t next = row[kFiRecOff] + row[kFiLines];
@@ -1113,9 +1115,11 @@ __global__ void __launch_bounds__(256, kBlocks)
           at = next;
         }
         if (at >= end) break;
+        k = uint32_t(at - base);
       }
-      const uint64_t r = at + uint32_t(g.shift / G);
-      bool pending = r < end;
+      const uint64_t r = base + k + uint32_t(g.shift / G);
+      bool pending = r < records;
+      if constexpr (kPart) pending = pending && r < base + chunk;
       uint64_t rec_off = 0, lines = 0;
       if (pending) {
         for (;; ++f) {  // the warp's later records may be in later files
@@ -1127,7 +1131,7 @@ __global__ void __launch_bounds__(256, kBlocks)
       const uint64_t *row = q.file_info + uint64_t(f) * kFileInfoWords;
       const IndexFile F = q.files[f];
       const uint32_t qid = group_of(q, row);
-      if (q.group_mask != 0) pending = pending && ((q.group_mask >> qid) & 1u) != 0;
+      if constexpr (kPart) pending = pending && ((q.group_mask >> qid) & 1u) != 0;
       const uint64_t i = r - rec_off;
       const int64_t *nl = q.NL + row[kFiNlOff];
       // batch files are below 2 GiB (int32 results): 32-bit positions
@@ -1238,14 +1242,14 @@ cudaError_t state_bytes(Kernel kernel, const QueryNeeds &needs, int block, size_
                               int(2 * kMaxQueryLevels * 256 * sizeof(Pos)));
 }
 
-template <int G, int kBlocks>
+template <int G, int kBlocks, bool kPart = false>
 cudaError_t batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
                               int grid, int block, cudaStream_t stream) {
   // A plain launch: blocks that start beside the indexer's last CTAs keep the
   // SM split for those (200 KB of shared memory, little L1) for as long as they
   // run (1,500 MiB of files: 1,371 us a replay instead of 1,213).
-  auto kernel = needs.ext ? batch_query_kernel<true, G, kBlocks>
-                          : batch_query_kernel<false, G, kBlocks>;
+  auto kernel = needs.ext ? batch_query_kernel<true, G, kBlocks, kPart>
+                          : batch_query_kernel<false, G, kBlocks, kPart>;
   size_t smem = 0;
   const cudaError_t e = state_bytes<int32_t>(kernel, needs, block, smem);
   if (e != cudaSuccess) return e;
@@ -1335,6 +1339,7 @@ BatchShape batch_shape(const BatchQueryLaunch &q, const QueryNeeds &needs, int g
   return s;
 }
 
+template <bool kPart>
 cudaError_t batch_query_part(const BatchQueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
                              int grid, int block, cudaStream_t stream) {
   const BatchShape s = batch_shape(q, needs, grid, block);
@@ -1342,11 +1347,13 @@ cudaError_t batch_query_part(const BatchQueryLaunch &q, const IrBlob &ir, const 
     const cudaError_t e = cudaMemsetAsync(q.record_counter, 0, sizeof(unsigned long long), stream);
     if (e != cudaSuccess) return e;
   }
-  if (s.lanes == 32) return batch_query_start<32, 4>(q, ir, needs, s.grid, block, stream);
-  if (s.lanes == 16) return batch_query_start<16, 4>(q, ir, needs, s.grid, block, stream);
-  if (s.lanes == 8) return batch_query_start<8, 4>(q, ir, needs, s.grid, block, stream);
-  return s.five ? batch_query_start<1, 5>(q, ir, needs, s.grid, block, stream)
-                : batch_query_start<1, 4>(q, ir, needs, s.grid, block, stream);
+  if (s.lanes == 32) return batch_query_start<32, 4, kPart>(q, ir, needs, s.grid, block, stream);
+  if constexpr (!kPart) {  // (a part has 32 lanes or one: descending_apart)
+    if (s.lanes == 16) return batch_query_start<16, 4>(q, ir, needs, s.grid, block, stream);
+    if (s.lanes == 8) return batch_query_start<8, 4>(q, ir, needs, s.grid, block, stream);
+  }
+  return s.five ? batch_query_start<1, 5, kPart>(q, ir, needs, s.grid, block, stream)
+                : batch_query_start<1, 4, kPart>(q, ir, needs, s.grid, block, stream);
 }
 
 cudaError_t query_part(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
@@ -1394,10 +1401,10 @@ int batch_query_grid(BatchQueryLaunch q, const IrBlob &ir, int grid, int block) 
 cudaError_t batch_query_launch(BatchQueryLaunch q, const IrBlob &ir, int grid, int block,
                                cudaStream_t stream) {
   const BatchParts parts(q, ir);
-  if (!parts.split) return batch_query_part(q, ir, parts.needs[0], grid, block, stream);
+  if (!parts.split) return batch_query_part<false>(q, ir, parts.needs[0], grid, block, stream);
   for (int d = 0; d < 2; ++d) {
     q.group_mask = parts.masks[d];
-    const cudaError_t e = batch_query_part(q, ir, parts.needs[d], grid, block, stream);
+    const cudaError_t e = batch_query_part<true>(q, ir, parts.needs[d], grid, block, stream);
     if (e != cudaSuccess) return e;
     q.counter_cleared = false;
   }

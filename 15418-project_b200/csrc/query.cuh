@@ -88,8 +88,8 @@ struct BatchQueryLaunch {
   int num_groups = 0;
   BatchQueryGroup groups[kMaxBatchGroups];
   uint32_t used_groups = ~0u;  // bit g: some file is of group g
-  // groups whose files' records the launch runs, 0 for all of them
-  // (batch_query_launch sets it)
+  // groups whose files' records a launch of some of them runs (batch_query_launch
+  // sets it)
   uint32_t group_mask = 0;
 };
 
