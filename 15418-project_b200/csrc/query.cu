@@ -398,8 +398,8 @@ struct Key {
 // One lane.  Does the string before the ':' at `colon` equal the key (the
 // test of MOVE_TO_KEY, query.cu:254-302)?  `s_word` is the string-mask word of
 // the byte before the colon.  Most keys differ in length or in their first
-// bytes: the quote and three bytes are compared as one word, from the one or
-// two aligned words that hold them.
+// bytes: the quote and three bytes are compared as one word, first as far as
+// the aligned word that holds the quote goes, then with the next one.
 template <typename Pos>
 __device__ __forceinline__ bool key_at_colon(const Rec<Pos> &c, const Query &q, Pos line_start,
                                              Pos colon, uint64_t s_word, const Key &key) {
@@ -415,6 +415,7 @@ __device__ __forceinline__ bool key_at_colon(const Rec<Pos> &c, const Query &q, 
   const uint32_t *word = reinterpret_cast<const uint32_t *>(addr & ~uintptr_t(3));
   const uint32_t shift = uint32_t(addr & 3u) * 8u;
   uint32_t head = word[0] >> shift;
+  if (((head ^ key.head) & key.mask & (0xFFFFFFFFu >> shift)) != 0) return false;
   // bytes up to the string's end only: the second word holds one of them
   if (shift != 0 && (key.mask >> (32 - shift)) != 0) head |= word[1] << (32 - shift);
   if (((head ^ key.head) & key.mask) != 0) return false;
@@ -429,13 +430,18 @@ __device__ __forceinline__ uint64_t string_word_before(const Rec<Pos> &c, Pos p)
 }
 
 // find_key (below) by one lane for its own record: one pair of characters a
-// step, their bytes and the string-mask word loaded together.
+// step, their bytes loaded together; several keys end in one string-mask word,
+// which is kept (1 M records of 512 bytes, 24 keys each, none the one looked
+// for: 256 us with the word loaded for every key, 237 so, 211 with the two-step
+// comparison of key_at_colon; posts, 131 K: 88, 84 and 82).
 template <typename Pos>
 __device__ __forceinline__ bool find_key_lane(const Rec<Pos> &c, const Query &q, Pos line_start,
                                               Pos level_end, const uint64_t *lvl, const Key &key,
                                               Pos &line_index, Pos &next, bool &open) {
   const Pos from = line_index + 1;
   Walk<Pos> walk(c, lvl, from, level_end);
+  Pos s_at = -1;
+  uint64_t s_word = 0;
   for (;;) {
     const Pos p1 = walk.next();
     if (p1 < 0 || p1 > level_end) return false;
@@ -443,8 +449,11 @@ __device__ __forceinline__ bool find_key_lane(const Rec<Pos> &c, const Query &q,
     if (p2 > level_end) p2 = -1;
     const uint8_t b1 = c.in[p1];
     const uint8_t b2 = p2 >= 0 ? c.in[p2] : uint8_t(0);
-    const uint64_t s = string_word_before(c, p1);
-    if (b1 != ':' || key_at_colon(c, q, line_start, p1, s, key)) {
+    if (((p1 - 1) >> 6) != s_at) {
+      s_at = (p1 - 1) >> 6;
+      s_word = c.S[s_at];
+    }
+    if (b1 != ':' || key_at_colon(c, q, line_start, p1, s_word, key)) {
       line_index = p1;
       next = p2;
       open = false;
@@ -710,20 +719,28 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
   if (line_end >= c.n) line_end = c.n - 1;
   // the record's braces: last '}' back from line_end, first '{' from
   // line_start, G bytes a round
-  for (bool need = alive; __any_sync(kAll, need);) {
-    const Pos p = line_end - g.lane;
-    const unsigned hit = g.ballot(need && (p <= line_start || at(c, p) == '}'));
-    if (need) {
-      line_end -= hit != 0 ? __ffs(int(hit)) - 1 : G;
-      need = hit == 0;
+  if constexpr (G == 1) {
+    if (alive) {
+      while (line_end > line_start && at(c, line_end) != '}') --line_end;
+      while (line_start < line_end && at(c, line_start) != '{') ++line_start;
     }
-  }
-  for (bool need = alive; __any_sync(kAll, need);) {
-    const bool past = line_end - line_start <= g.lane;
-    const unsigned hit = g.ballot(need && (past || at(c, Pos(line_start + g.lane)) == '{'));
-    if (need) {
-      line_start += hit != 0 ? __ffs(int(hit)) - 1 : G;
-      need = hit == 0;
+    __syncwarp();
+  } else {
+    for (bool need = alive; __any_sync(kAll, need);) {
+      const Pos p = line_end - g.lane;
+      const unsigned hit = g.ballot(need && (p <= line_start || at(c, p) == '}'));
+      if (need) {
+        line_end -= hit != 0 ? __ffs(int(hit)) - 1 : G;
+        need = hit == 0;
+      }
+    }
+    for (bool need = alive; __any_sync(kAll, need);) {
+      const bool past = line_end - line_start <= g.lane;
+      const unsigned hit = g.ballot(need && (past || at(c, Pos(line_start + g.lane)) == '{'));
+      if (need) {
+        line_start += hit != 0 ? __ffs(int(hit)) - 1 : G;
+        need = hit == 0;
+      }
     }
   }
   alive = alive && line_start < line_end;
