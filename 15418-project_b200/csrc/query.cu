@@ -1384,9 +1384,13 @@ cudaError_t query_start(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds
 // 113, 128 and 160; 349 K: 165, 145 and 182.  (Full waves of $.user.lang on
 // posts take 76, 98 and 126 us, a little more than 4 : 5 : 6.  By those weights
 // 606 to 682 K records would take four blocks instead of six, which array
-// elements want, 265 us for 290, and posts do not, 366 for 338.)
+// elements want, 265 us for 290, and posts do not, 366 for 338.)  Many waves
+// overlap, and from twenty blocks per SM on five are the better of four and
+// five: 1 M records of 512 bytes 221 us, 229 with four; 3 M of 32 bytes 113 and
+// 120; 850 K posts 416 and 429, array elements 321 and 318.
 int blocks_per_sm(uint64_t records) {
   const uint64_t per_block = resident_threads() / 4u;  // one block on every SM
+  if (records > 20u * per_block) return 5;
   int best = 4;
   uint64_t best_cost = ~uint64_t(0);
   for (int b : {4, 5, 6}) {
