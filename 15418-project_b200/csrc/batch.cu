@@ -48,6 +48,7 @@ struct gpj_batch {
   int32_t *d_out = nullptr;
   uint64_t *d_info = nullptr, *d_totals = nullptr;
   void *d_scratch = nullptr;
+  uint64_t file_bytes = 0;  // of all files
   uint64_t s_words = 0, lb_words = 0, nl_slots = 0, result_ints = 0, records = 0;
   // launch shape
   int index_threads = gpjb::kIndexThreads;
@@ -136,6 +137,7 @@ gpjb::BatchQueryLaunch query_launch_of(const gpj_batch *b, bool after_index) {
   q.status = reinterpret_cast<unsigned int *>(b->d_totals + gpjb::kTotError);
   q.record_counter = reinterpret_cast<unsigned long long *>(b->d_totals + gpjb::kTotRecordCounter);
   q.expected_records = b->records;
+  q.expected_bytes = b->file_bytes;
   q.num_groups = int(b->groups.size());
   for (size_t g = 0; g < b->groups.size(); ++g) q.groups[g] = b->groups[g];
   q.used_groups = b->used_groups;
@@ -298,6 +300,7 @@ int gpj_batch_create(gpj_ctx *ctx, const uint8_t *d_input, uint64_t input_bytes,
     }
     b->files[f].in_off = bf.offset;
     b->files[f].n = bf.size_bytes;
+    b->file_bytes += bf.size_bytes;
     b->files[f].levels = int32_t(queries[bf.query].num_levels);
     b->query_of_file[f] = bf.query;
     b->used_groups |= 1u << bf.query;

@@ -682,88 +682,124 @@ __device__ bool find_key(const Rec<Pos> &c, const Query &q, const Group<G> &g, b
   return found;
 }
 
-// "..name" by a whole warp: every member named key inside (line_index,
-// level_end), at any level from `level` up, in document order (by the position
-// of its ':').  The lanes list the structural characters of all those levels
-// in their words, test one each for the key, and collect the few that match;
-// those are then resolved one per lane.  (Each lane testing the characters of
-// its own word left two thirds of the lanes idle: 41 K records 231 us, so 200.)
-// Returns `stored` plus the matches.
+// One lane.  Stores the member whose ':' is at p, `level` or a level above it.
 template <typename Pos, typename OutT>
-__device__ int descend(const Rec<Pos> &c, const Query &q, const Group<32> &g, Pos line_start,
-                       Pos line_index, Pos level_end, int level, const Key &key, int stored,
-                       OutT *out, uint16_t *list, Pos *matches) {
-  int waiting = 0;  // collected matches
-  auto resolve = [&] {
-    __syncwarp();
-    if (g.lane < waiting) {
-      const Pos p = matches[g.lane];
-      const int slot = stored + g.lane;
-      if (slot >= q.num_results) {
-        raise_status(c, kQueryStatusOverflow);
-      } else {
-        int l = level;
-        while (l < c.levels && (level_words(c, l) == nullptr ||
-                                ((level_words(c, l)[p >> 6] >> (p & 63)) & 1ull) == 0ull))
-          ++l;
-        const Pos vend = next_struct_lane(c, level_end, Pos(p + 1), level_words(c, l));
-        Pos vs = p + 1;
-        while (at(c, vs) == ' ' && vs < vend) ++vs;
-        Pos ve = vend;
-        while (ve > vs && at(c, ve - 1) == ' ') --ve;
-        out[2 * slot] = OutT(vs);
-        out[2 * slot + 1] = OutT(ve);
-      }
-    }
-    stored += waiting;
-    waiting = 0;
-    __syncwarp();
-  };
+__device__ __forceinline__ void store_member(const Rec<Pos> &c, const Query &q, Pos level_end,
+                                             int level, Pos p, int slot, OutT *out) {
+  if (slot >= q.num_results) {
+    raise_status(c, kQueryStatusOverflow);
+    return;
+  }
+  int l = level;
+  while (l < c.levels && (level_words(c, l) == nullptr ||
+                          ((level_words(c, l)[p >> 6] >> (p & 63)) & 1ull) == 0ull))
+    ++l;
+  const Pos vend = next_struct_lane(c, level_end, Pos(p + 1), level_words(c, l));
+  Pos vs = p + 1;
+  while (at(c, vs) == ' ' && vs < vend) ++vs;
+  Pos ve = vend;
+  while (ve > vs && at(c, ve - 1) == ' ') --ve;
+  out[2 * slot] = OutT(vs);
+  out[2 * slot + 1] = OutT(ve);
+}
+
+// The structural characters of word w at any level from `lowest` up, in
+// [line_index, level_end).
+template <typename Pos>
+__device__ __forceinline__ uint64_t any_level_word(const Rec<Pos> &c, int lowest, Pos w,
+                                                   Pos line_index, Pos level_end) {
+  uint64_t cand = 0;
+  const uint64_t *row = c.LB + uint64_t(c.W) * uint64_t(lowest) + w;
+#pragma unroll 4
+  for (int l = lowest; l < c.levels; ++l, row += c.W) cand |= *row;
+  if (w == (line_index >> 6)) cand &= ~0ull << (line_index & 63);
+  if (w == (level_end >> 6)) cand &= (1ull << (level_end & 63)) - 1ull;
+  return cand;
+}
+
+// "..name": every member named key inside (line_index, level_end), at any level
+// from `level` up, in document order (by the position of its ':'), for every
+// active record of the warp.  The lanes of a group list the structural
+// characters of all those levels in their words, test one each for the key, and
+// collect the few that match; those are then resolved one per lane.  (Each lane
+// testing the characters of its own word left two thirds of the lanes idle:
+// 41 K posts 231 us, so 200.)  One lane tests them one after another.  Returns
+// `stored` plus the record's matches.
+template <typename Pos, typename OutT, int G>
+__device__ int descend(const Rec<Pos> &c, const Query &q, const Group<G> &g, bool active,
+                       Pos line_start, Pos line_index, Pos level_end, int level, const Key &key,
+                       int stored, OutT *out, uint16_t *list, Pos *matches) {
   const int lowest = level > 0 ? level : 0;
   const Pos last = min(Pos((level_end - 1) >> 6), Pos(c.W - 1));
-  for (Pos w0 = line_index >> 6; w0 <= last;) {
-    const Pos w = w0 + g.lane;
-    uint64_t cand = 0, s_word = 0;
-    if (w >= 0 && w <= last) {
-      const uint64_t *row = c.LB + uint64_t(c.W) * uint64_t(lowest) + w;
-#pragma unroll 4
-      for (int l = lowest; l < c.levels; ++l, row += c.W) cand |= *row;
-      s_word = c.S[w];
-      if (w == (line_index >> 6)) cand &= ~0ull << (line_index & 63);
-      if (w == (level_end >> 6)) cand &= (1ull << (level_end & 63)) - 1ull;
+  Pos w0 = line_index >> 6;
+  if constexpr (G == 1) {
+    if (active) {
+      for (Pos w = max(w0, Pos(0)); w <= last; ++w) {
+        uint64_t cand = any_level_word(c, lowest, w, line_index, level_end);
+        const uint64_t s_word = cand != 0 ? c.S[w] : 0ull;
+        for (; cand != 0; cand &= cand - 1) {
+          const Pos p = w * 64 + __ffsll(static_cast<long long>(cand)) - 1;
+          if (c.in[p] == ':' &&
+              key_at_colon(c, q, line_start, p, (p & 63) != 0 ? s_word : string_word_before(c, p),
+                           key))
+            store_member(c, q, level_end, level, p, stored++, out);
+        }
+      }
     }
-    const int mine = __popcll(cand);
-    int total;
-    int at_slot = g.sum_before(mine, total);
-    int words = 32;
-    if (total > kListed<32>) {
-      words = __popc(g.ballot(g.lane == 0 || at_slot + mine <= kListed<32>));
-      total = g.shfl(at_slot + mine, words - 1);
-    }
-    if (g.lane < words) list_bits(list + at_slot, cand, g.lane * 64);
     __syncwarp();
-    const Pos base = w0 * 64;
-    const uint8_t *text = c.in + base;
-    for (int e0 = 0; e0 < total; e0 += 32) {
-      const bool has = e0 + g.lane < total;
-      const int o = has ? int(list[e0 + g.lane]) : 0;
-      const uint8_t b = has ? text[o] : uint8_t(0);
-      uint64_t s = __shfl_sync(kAll, (unsigned long long)s_word, (o - 1) >> 6);
-      if (has && o == 0) s = string_word_before(c, base);
-      const bool match =
-          b == ':' && key_at_colon(c, q, line_start, Pos(base + o), s, key);
+    return stored;
+  } else {
+    int waiting = 0;  // collected matches
+    auto resolve = [&] {
       __syncwarp();
-      const unsigned hits = g.ballot(match);
-      if (hits == 0) continue;
-      if (waiting + __popc(hits) > 32) resolve();
-      if (match) matches[waiting + __popc(hits & ((1u << g.lane) - 1u))] = base + o;
-      waiting += __popc(hits);
+      if (g.lane < waiting)
+        store_member(c, q, level_end, level, matches[g.lane], stored + g.lane, out);
+      stored += waiting;
+      waiting = 0;
+      __syncwarp();
+    };
+    bool need = active && w0 <= last;
+    while (__any_sync(kAll, need)) {
+      const Pos w = w0 + g.lane;
+      const bool have = need && w >= 0 && w <= last;
+      const uint64_t cand = have ? any_level_word(c, lowest, w, line_index, level_end) : 0ull;
+      const uint64_t s_word = have ? c.S[w] : 0ull;
+      const int mine = __popcll(cand);
+      int total;
+      const int at_slot = g.sum_before(mine, total);
+      int words = G;
+      if (__any_sync(kAll, total > kListed<G>)) {
+        words = __popc(g.ballot(g.lane == 0 || at_slot + mine <= kListed<G>));
+        total = g.shfl(at_slot + mine, words - 1);
+      }
+      if (g.lane < words) list_bits(list + at_slot, cand, g.lane * 64);
+      __syncwarp();
+      const Pos base = w0 * 64;
+      const uint8_t *text = c.in + base;
+      for (int e0 = 0; __any_sync(kAll, e0 < total); e0 += G) {
+        const bool has = e0 + g.lane < total;
+        const int o = has ? int(list[e0 + g.lane]) : 0;
+        const uint8_t b = has ? text[o] : uint8_t(0);
+        uint64_t s = __shfl_sync(kAll, (unsigned long long)s_word, (o - 1) >> 6, G);
+        if (has && o == 0) s = string_word_before(c, base);
+        const bool match = b == ':' && key_at_colon(c, q, line_start, Pos(base + o), s, key);
+        __syncwarp();
+        const unsigned hits = g.ballot(match);
+        const int found = __popc(hits);
+        if (!__any_sync(kAll, found != 0)) continue;
+        if (__any_sync(kAll, waiting + found > G)) resolve();
+        if (match) matches[waiting + __popc(hits & ((1u << g.lane) - 1u))] = base + o;
+        waiting += found;
+      }
+      if (need) {
+        w0 += words;
+        need = w0 <= last;
+      }
+      __syncwarp();
     }
-    w0 += words;
-    __syncwarp();
+    resolve();
+    return stored;
   }
-  resolve();
-  return stored;
 }
 
 // One lane.  Commas among the structural characters after line_index, up to
@@ -781,13 +817,19 @@ __device__ int count_commas(const Rec<Pos> &c, Steps<Pos> max_steps, Pos level_e
   return commas;
 }
 
+// Opcodes an instance of the kernels runs: the reference's; with the numeric
+// filters and the element checks of "[*]" and the open slices; with "..name"
+// too.
+enum : int { kReference = 0, kExtensions = 1, kDescends = 2 };
+
 // Runs the query over the warp's records (one per group of G lanes; `alive`:
 // the group has one).  `ends` and `marks` are the thread's slots of per-level
 // and per-mark positions in shared memory ([level * stride]).
-template <typename Pos, typename OutT, bool kExt, int G>
+template <typename Pos, typename OutT, int kOps, int G>
 __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g, bool alive,
                             Pos line_start, Pos line_end, OutT *out, Pos *ends, Pos *marks,
                             int stride, uint16_t *list, Pos *matches) {
+  constexpr bool kExt = kOps >= kExtensions;
   // every lane keeps its own copy of its record's state, so no lane reads
   // what another wrote, except the result slots
   if (alive)
@@ -1061,17 +1103,15 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       break;
     }
     case OP_DESCEND_KEY: {
-      // (lanes_per_record gives IR with this opcode a whole warp)
-      if constexpr (!kExt || G != 32) {
+      if constexpr (kOps < kDescends) {
         return;
       } else {
         const int key_len = read_varint(q, qp, operand);
         const int key_pos = qp;
         if (key_len < 0 || !LEVEL_OK(level)) return;
         qp = ir_skip(q.ir_len, qp, key_len);
-        if (alive)
-          stored = descend(c, q, g, line_start, line_index, ends[level * stride], q.base + level,
-                           Key(q, key_pos, key_len), stored, out, list, matches);
+        stored = descend(c, q, g, alive, line_start, line_index, ends[level * stride],
+                         q.base + level, Key(q, key_pos, key_len), stored, out, list, matches);
         break;
       }
     }
@@ -1114,17 +1154,15 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
 #undef LEVEL_OK
 }
 
-// kExt: the IR holds extension opcodes (numeric filters, "..name", the
-// element checks of "[*]" and the open slices); reference-syntax IR runs the
-// variant without them.
+// kOps: the opcodes of the IR of the launch's queries.
 // kBlocks: 256-thread blocks per SM that the registers are held to.
-template <typename Pos, typename OutT, bool kExt, int G, int kBlocks>
+template <typename Pos, typename OutT, int kOps, int G, int kBlocks>
 __global__ void __launch_bounds__(256, kBlocks)
     query_kernel(const __grid_constant__ QueryLaunch q, const __grid_constant__ IrBlob ir,
                  int nlev, int max_marks) {
   __shared__ __align__(16) uint8_t s_ir[kMaxQueryIrBytes + kIrPad];
   __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed<G>];
-  __shared__ Pos s_match[kExt && G == 32 ? 8 : 1][32];
+  __shared__ Pos s_match[kOps == kDescends && G > 1 ? 256 / G : 1][G];
   extern __shared__ __align__(8) uint8_t s_state[];  // Pos[nlev + marks][bdim]
   const QueryOne &one = q.queries[blockIdx.y];
   for (int i = threadIdx.x; i < one.ir_len + kIrPad; i += blockDim.x)
@@ -1143,10 +1181,10 @@ __global__ void __launch_bounds__(256, kBlocks)
     const bool alive = r < q.num_lines;
     const int64_t start = alive ? q.NL[r] : 0;
     const int64_t end = alive && r + 1 < q.num_lines ? q.NL[r + 1] : q.n - 1;
-    run_records<Pos, OutT, kExt, G>(c, query, g, alive, Pos(start), Pos(end),
+    run_records<Pos, OutT, kOps, G>(c, query, g, alive, Pos(start), Pos(end),
                                     out + r * int64_t(one.num_results) * 2, ends, marks,
                                     int(blockDim.x), s_list[G > 1 ? threadIdx.x / G : 0],
-                                    s_match[kExt && G == 32 ? threadIdx.x / 32 : 0]);
+                                    s_match[kOps == kDescends && G > 1 ? threadIdx.x / G : 0]);
     __syncwarp();
   }
 }
@@ -1173,7 +1211,7 @@ __device__ __forceinline__ uint32_t group_of(const BatchQueryLaunch &q, const ui
 }
 
 // kPart: the launch runs the records of some groups' files only (group_mask).
-template <bool kExt, int G, int kBlocks, bool kPart>
+template <int kOps, int G, int kBlocks, bool kPart>
 __global__ void __launch_bounds__(256, kBlocks)
     batch_query_kernel(const BatchQueryLaunch q, const __grid_constant__ IrBlob ir, int nlev,
                        int max_marks) {
@@ -1190,7 +1228,7 @@ __global__ void __launch_bounds__(256, kBlocks)
   }
   __syncthreads();
   __shared__ uint16_t s_list[G > 1 ? 256 / G : 1][kListed<G>];
-  __shared__ int32_t s_match[kExt && G == 32 ? 8 : 1][32];
+  __shared__ int32_t s_match[kOps == kDescends && G > 1 ? 256 / G : 1][G];
   const Group<G> g;
   int32_t *ends = reinterpret_cast<int32_t *>(s_state) + threadIdx.x;
   int32_t *marks = ends + nlev * blockDim.x;
@@ -1253,11 +1291,11 @@ __global__ void __launch_bounds__(256, kBlocks)
         const BatchQueryGroup grp = q.groups[now];
         const Query query{s_ir + s_ir_off[now], grp.ir_len, grp.num_results, grp.base_level, nlev,
                           max_marks, grp.ext};
-        run_records<int32_t, int32_t, kExt, G>(
+        run_records<int32_t, int32_t, kOps, G>(
             c, query, g, mine, start, end,
             q.out + row[kFiOutOff] + i * uint64_t(grp.num_results) * 2u, ends, marks,
             int(blockDim.x), s_list[G > 1 ? threadIdx.x / G : 0],
-            s_match[kExt && G == 32 ? threadIdx.x / 32 : 0]);
+            s_match[kOps == kDescends && G > 1 ? threadIdx.x / G : 0]);
         __syncwarp();
         pending = pending && !mine;
       }
@@ -1303,13 +1341,30 @@ uint64_t resident_threads() {
 // / 293 (140).  Where one lane begins to win depends on the IR, at which the
 // rule does not look: its line (19 K records) lies between the short IR's, which
 // loses 6 us at 28 K by it, and the eight-slot one's, which gains 50 there.
+// Records of one bitmap word on average take one lane at any count: there is
+// nothing to share (15 K records of 32 bytes with a numeric filter: 13 us, 16.6
+// with 8 lanes).
+//
 // "..name" reads every level's words of the whole record, which only a wide
-// group reads in whole sectors: 41 K records 897 us with one lane of this
-// kernel, 293 with 8, 231 with 32 (200 with the search of descend).
-int lanes_per_record(uint64_t records, bool descends) {
-  if (descends) return 32;
-  if (records == 0) return 1;
+// group reads in whole sectors: 41 K posts of 2,400 bytes 897 us with one lane,
+// 293 with 8, 231 with 32 (200 with the search of descend).  Shorter records
+// leave its lanes idle (us, 32 / 8 / one lane, one thread per record before this
+// split in brackets): 2 M of 8 bytes 2,061 / 516 / 89 (92), of 128 bytes 2,455 /
+// 667 / 237 (249); 300 K of 512 bytes, all alike, 419 / 138 / 95 (112), 256 K of
+// 422 bytes, mixed, 632 / 485 / 589 (700); 15 K of 1,024 bytes 26 / 15 / 30 (40),
+// 60 K 84 / 41 / 49 (59).  From 2 KiB on mixed records, as posts are, win more
+// by 32 lanes (240 K of 2.4 KB 746 / 860 / 2,997 (2,967)) than records all alike
+// lose (200 K 476 (434)).
+int lanes_per_record(uint64_t records, uint64_t bytes, bool descends) {
+  if (records == 0) return descends ? 32 : 1;
   const uint64_t threads = resident_threads();
+  const uint64_t mean = bytes / records;
+  if (descends) {
+    if (records * 32u <= threads) return 32;
+    if (mean <= 1024u) return records * 8u <= threads ? 8 : 1;
+    return mean <= 2048u ? 8 : 32;
+  }
+  if (mean <= 64u) return 1;
   for (int g : {32, 16, 8})
     if (records * uint64_t(g) <= threads) return g;
   return 1;
@@ -1321,7 +1376,9 @@ int lanes_per_record(uint64_t records, bool descends) {
 // small file asks "..id": query stage 5,696 us together, 1,318 apart).  Up to
 // there a launch of each after the other takes longer (1.5 K records: 35 and 54
 // us; 14 K runs in a host call: 290 and 327).
-bool descending_apart(uint64_t records) { return lanes_per_record(records, false) == 1; }
+bool descending_apart(uint64_t records, uint64_t bytes) {
+  return lanes_per_record(records, bytes, false) == 1;
+}
 
 // What the queries of a launch need together.
 struct QueryNeeds : IrNeeds {
@@ -1345,14 +1402,23 @@ cudaError_t state_bytes(Kernel kernel, const QueryNeeds &needs, int block, size_
                               int(2 * kMaxQueryLevels * 256 * sizeof(Pos)));
 }
 
+// "..name" runs with 32, 8 or 1 lanes (lanes_per_record), the last without a
+// choice of blocks per SM.
+template <int G, int kBlocks>
+constexpr bool descending_instance() {
+  return G == 32 || G == 8 || (G == 1 && kBlocks <= 4);
+}
+
 template <int G, int kBlocks, bool kPart = false>
 cudaError_t batch_query_start(const BatchQueryLaunch &q, const IrBlob &ir, const QueryNeeds &needs,
                               int grid, int block, cudaStream_t stream) {
   // A plain launch: blocks that start beside the indexer's last CTAs keep the
   // SM split for those (200 KB of shared memory, little L1) for as long as they
   // run (1,500 MiB of files: 1,371 us a replay instead of 1,213).
-  auto kernel = needs.ext ? batch_query_kernel<true, G, kBlocks, kPart>
-                          : batch_query_kernel<false, G, kBlocks, kPart>;
+  auto kernel = needs.ext ? batch_query_kernel<kExtensions, G, kBlocks, kPart>
+                          : batch_query_kernel<kReference, G, kBlocks, kPart>;
+  if constexpr (descending_instance<G, kBlocks>())
+    if (needs.descends) kernel = batch_query_kernel<kDescends, G, kBlocks, kPart>;
   size_t smem = 0;
   const cudaError_t e = state_bytes<int32_t>(kernel, needs, block, smem);
   if (e != cudaSuccess) return e;
@@ -1367,8 +1433,10 @@ cudaError_t query_start(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds
   const dim3 grid(
       unsigned(std::min<int64_t>((q.num_lines + per_block - 1) / per_block, 0x7FFFFFFF)),
       unsigned(q.num_queries));
-  auto kernel = needs.ext ? query_kernel<Pos, OutT, true, G, kBlocks>
-                          : query_kernel<Pos, OutT, false, G, kBlocks>;
+  auto kernel = needs.ext ? query_kernel<Pos, OutT, kExtensions, G, kBlocks>
+                          : query_kernel<Pos, OutT, kReference, G, kBlocks>;
+  if constexpr (descending_instance<G, kBlocks>())
+    if (needs.descends) kernel = query_kernel<Pos, OutT, kDescends, G, kBlocks>;
   size_t smem = 0;
   const cudaError_t e = state_bytes<Pos>(kernel, needs, block, smem);
   if (e != cudaSuccess) return e;
@@ -1410,7 +1478,7 @@ cudaError_t query_start_narrow(const QueryLaunch &q, const IrBlob &ir, const Que
   if (lanes == 32) return query_start<int32_t, OutT, 32, 4>(q, ir, needs, block, stream);
   if (lanes == 16) return query_start<int32_t, OutT, 16, 4>(q, ir, needs, block, stream);
   if (lanes == 8) return query_start<int32_t, OutT, 8, 4>(q, ir, needs, block, stream);
-  switch (blocks_per_sm(runs)) {
+  switch (needs.descends ? 4 : blocks_per_sm(runs)) {
   case 5: return query_start<int32_t, OutT, 1, 5>(q, ir, needs, block, stream);
   case 6: return query_start<int32_t, OutT, 1, 6>(q, ir, needs, block, stream);
   default: return query_start<int32_t, OutT, 1, 4>(q, ir, needs, block, stream);
@@ -1424,7 +1492,7 @@ struct BatchShape {
   bool five = false;
 };
 BatchShape batch_shape(const BatchQueryLaunch &q, const QueryNeeds &needs, int grid, int block) {
-  BatchShape s{lanes_per_record(q.expected_records, needs.descends), grid};
+  BatchShape s{lanes_per_record(q.expected_records, q.expected_bytes, needs.descends), grid};
   if (q.expected_records > 0) {
     const uint64_t blocks = (q.expected_records * uint64_t(s.lanes) + uint64_t(block) - 1) / block;
     s.grid = int(std::min<uint64_t>(uint64_t(grid), blocks));
@@ -1436,7 +1504,7 @@ BatchShape batch_shape(const BatchQueryLaunch &q, const QueryNeeds &needs, int g
   // with six; 216 K: 162 and 179; 588 K: 316 and 327 with five; 3.8 M: 1.62 ms
   // and 1.94 with six).
   const uint64_t one_each = resident_threads() / 4u;  // records of a block on every SM
-  s.five = q.expected_records > 4u * one_each && q.expected_records <= 5u * one_each;
+  s.five = !needs.descends && q.expected_records > 4u * one_each && q.expected_records <= 5u * one_each;
   // Runs taken from the counter want no blocks beyond the resident ones: a
   // later block's first run is its own and waits for it (192 K records: 169 us
   // with eight blocks per SM in the grid, 155 with four; 274 K: 193 and 181).
@@ -1455,10 +1523,9 @@ cudaError_t batch_query_part(const BatchQueryLaunch &q, const IrBlob &ir, const 
     if (e != cudaSuccess) return e;
   }
   if (s.lanes == 32) return batch_query_start<32, 4, kPart>(q, ir, needs, s.grid, block, stream);
-  if constexpr (!kPart) {  // (a part has 32 lanes or one: descending_apart)
+  if constexpr (!kPart)  // (a part has 32 lanes, 8 or one: descending_apart)
     if (s.lanes == 16) return batch_query_start<16, 4>(q, ir, needs, s.grid, block, stream);
-    if (s.lanes == 8) return batch_query_start<8, 4>(q, ir, needs, s.grid, block, stream);
-  }
+  if (s.lanes == 8) return batch_query_start<8, 4, kPart>(q, ir, needs, s.grid, block, stream);
   return s.five ? batch_query_start<1, 5, kPart>(q, ir, needs, s.grid, block, stream)
                 : batch_query_start<1, 4, kPart>(q, ir, needs, s.grid, block, stream);
 }
@@ -1468,13 +1535,14 @@ cudaError_t query_part(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds 
   constexpr int kBlock = 256;
   // the queries of a launch are resident side by side
   const uint64_t runs = uint64_t(q.num_lines) * uint64_t(q.num_queries);
-  const int lanes = lanes_per_record(runs, needs.descends);
+  const int lanes = lanes_per_record(runs, uint64_t(q.n) * uint64_t(q.num_queries), needs.descends);
   // partitions below 2 GiB take 32-bit positions whatever the result width
   // (700 MiB of posts, eight int64 slots: 427 us, 513 us before)
   if (!q.wide) return query_start_narrow<int32_t>(q, ir, needs, lanes, runs, kBlock, stream);
   if (q.n <= 0x7FFFFFFF)
     return query_start_narrow<int64_t>(q, ir, needs, lanes, runs, kBlock, stream);
-  if (lanes == 32) return query_start<int64_t, int64_t, 32, 3>(q, ir, needs, kBlock, stream);
+  if (lanes == 32 || (lanes > 1 && needs.descends))
+    return query_start<int64_t, int64_t, 32, 3>(q, ir, needs, kBlock, stream);
   return query_start<int64_t, int64_t, 1, 3>(q, ir, needs, kBlock, stream);
 }
 
@@ -1493,7 +1561,7 @@ struct BatchParts {
       needs[one.descends].add(one);
       masks[one.descends] |= 1u << g;
     }
-    split = masks[0] != 0 && masks[1] != 0 && descending_apart(q.expected_records);
+    split = masks[0] != 0 && masks[1] != 0 && descending_apart(q.expected_records, q.expected_bytes);
     if (!split) needs[0].add(needs[1]);
   }
 };
@@ -1531,7 +1599,8 @@ cudaError_t query_launch(QueryLaunch q, const IrBlob &ir, cudaStream_t stream) {
     needs[one.descends].add(one);
   }
   const bool split = parts[0].num_queries > 0 && parts[1].num_queries > 0 &&
-                     descending_apart(uint64_t(q.num_lines) * uint64_t(q.num_queries));
+                     descending_apart(uint64_t(q.num_lines) * uint64_t(q.num_queries),
+                                      uint64_t(q.n) * uint64_t(q.num_queries));
   if (!split) {
     needs[0].add(needs[1]);
     return query_part(q, ir, needs[0], stream);

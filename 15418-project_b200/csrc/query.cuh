@@ -82,9 +82,10 @@ struct BatchQueryLaunch {
   // strides)
   unsigned long long *record_counter = nullptr;
   bool counter_cleared = false;
-  // about the number of records (0: unknown, many): chooses the lanes per
-  // record and bounds the grid; the results do not depend on it
-  uint64_t expected_records = 0;
+  // about the number of records (0: unknown, many) and their bytes: choose the
+  // lanes per record, the number bounds the grid; the results do not depend on
+  // them
+  uint64_t expected_records = 0, expected_bytes = 0;
   int num_groups = 0;
   BatchQueryGroup groups[kMaxBatchGroups];
   uint32_t used_groups = ~0u;  // bit g: some file is of group g

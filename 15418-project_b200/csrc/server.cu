@@ -947,7 +947,7 @@ struct gpj_server {
     auto *d_files = reinterpret_cast<gpjb::IndexFile *>(dptr(b->meta_off));
     auto *d_rows = reinterpret_cast<uint64_t *>(dptr(b->meta_off + files_bytes));
     auto *d_stat = reinterpret_cast<unsigned int *>(dptr(b->meta_off + files_bytes + rows_bytes));
-    uint64_t records = 0;
+    uint64_t records = 0, bytes = 0;
     for (uint64_t v = 0; v < V; ++v) {
       const Pair &pr = pairs[v];
       Request *r = pr.r;
@@ -975,6 +975,7 @@ struct gpj_server {
       row[gpjb::kFiBytes] = res->size;
       row[gpjb::kFiQuery] = pr.group;
       records += bq.num_result_slots > 0 ? res->lines : 0u;
+      bytes += bq.num_result_slots > 0 ? res->size : 0u;
       if (bq.num_result_slots == 0) row[gpjb::kFiLines] = 0;
     }
     uint64_t *h_tot = h_rows + V * 8u;
@@ -1014,6 +1015,7 @@ struct gpj_server {
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg.device);
     ql.expected_records = records;
+    ql.expected_bytes = bytes;
     if (e == cudaSuccess && records > 0)
       e = gpjb::batch_query_launch(ql, blob, std::max(sms, 1) * 8, 128, s0.stream);
     b->refs = int(in_batch.size());
