@@ -1341,9 +1341,8 @@ uint64_t resident_threads() {
 // / 293 (140).  Where one lane begins to win depends on the IR, at which the
 // rule does not look: its line (19 K records) lies between the short IR's, which
 // loses 6 us at 28 K by it, and the eight-slot one's, which gains 50 there.
-// Records of one bitmap word on average take one lane at any count: there is
-// nothing to share (15 K records of 32 bytes with a numeric filter: 13 us, 16.6
-// with 8 lanes).
+// Records of one bitmap word on average skip 16 and 8 lanes: there is nothing to
+// share (15 K records of 32 bytes with a numeric filter: 13 us, 16.6 with 8).
 //
 // "..name" reads every level's words of the whole record, which only a wide
 // group reads in whole sectors: 41 K posts of 2,400 bytes 897 us with one lane,
@@ -1359,13 +1358,13 @@ int lanes_per_record(uint64_t records, uint64_t bytes, bool descends) {
   if (records == 0) return descends ? 32 : 1;
   const uint64_t threads = resident_threads();
   const uint64_t mean = bytes / records;
+  if (records * 32u <= threads) return 32;
   if (descends) {
-    if (records * 32u <= threads) return 32;
     if (mean <= 1024u) return records * 8u <= threads ? 8 : 1;
     return mean <= 2048u ? 8 : 32;
   }
   if (mean <= 64u) return 1;
-  for (int g : {32, 16, 8})
+  for (int g : {16, 8})
     if (records * uint64_t(g) <= threads) return g;
   return 1;
 }

@@ -58,15 +58,15 @@ def _data(count, mean):
 def _lanes(count, size, descends):
     threads = torch.cuda.get_device_properties(0).multi_processor_count * 1024
     mean = size // count
+    if count * 32 <= threads:
+        return 32
     if descends:
-        if count * 32 <= threads:
-            return 32
         if mean <= 1024:
             return 8 if count * 8 <= threads else 1
         return 8 if mean <= 2048 else 32
     if mean <= 64:
         return 1
-    return next((g for g in (32, 16, 8) if count * g <= threads), 1)
+    return next((g for g in (16, 8) if count * g <= threads), 1)
 
 
 QUERIES = [("$..k", 3), ("$.k..key", 2), ("$.k", 0), ("$.k[?(@.k >= 1)].k", 0)]
