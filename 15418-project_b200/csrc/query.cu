@@ -963,12 +963,16 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       const Pos lend = ends[level * stride];
       const uint64_t *lvl = level_words(c, q.base + level);
       Steps<Pos> steps = 0;
+      bool walked = false;  // this lane stands on the target already
       if constexpr (G == 1) {
-        if (alive)
+        if (alive) {
           alive = step_forward(c, max_steps, lend, lvl, target, line_index, ci, steps);
+          walked = ci == target;
+          if (walked) alive = alive && steps < max_steps;
+        }
         __syncwarp();
       }
-      for (bool run = alive; __any_sync(kAll, run);) {
+      for (bool run = alive && !walked; __any_sync(kAll, run);) {
         bool forward = false, back = false;
         if (run) {
           alive = ++steps <= max_steps;
@@ -1010,11 +1014,16 @@ __device__ void run_records(const Rec<Pos> &c, const Query &q, const Group<G> &g
       int32_t ci = ch == ']' ? 0 : current + 1;
       const uint64_t *lvl = level_words(c, q.base + level);
       Steps<Pos> steps = 0;
+      bool walked = false;  // this lane stands on the target already
       if constexpr (G == 1) {
-        if (alive) alive = step_backward(c, max_steps, lvl, target, line_index, ci, steps);
+        if (alive) {
+          alive = step_backward(c, max_steps, lvl, target, line_index, ci, steps);
+          walked = ci == target;
+          if (walked) alive = alive && steps < max_steps;
+        }
         __syncwarp();
       }
-      for (bool run = alive; __any_sync(kAll, run);) {
+      for (bool run = alive && !walked; __any_sync(kAll, run);) {
         bool forward = false, back = false;
         if (run) {
           alive = ++steps <= max_steps;
@@ -1542,7 +1551,9 @@ cudaError_t query_part(const QueryLaunch &q, const IrBlob &ir, const QueryNeeds 
     return query_start_narrow<int64_t>(q, ir, needs, lanes, runs, kBlock, stream);
   if (lanes == 32 || (lanes > 1 && needs.descends))
     return query_start<int64_t, int64_t, 32, 3>(q, ir, needs, kBlock, stream);
-  return query_start<int64_t, int64_t, 1, 3>(q, ir, needs, kBlock, stream);
+  // (four blocks per SM, 60 registers: 2.3 GiB of posts, one path 515 us, 588 with
+  // the 69 registers of three; eight slots 1,229 and 1,330)
+  return query_start<int64_t, int64_t, 1, 4>(q, ir, needs, kBlock, stream);
 }
 
 // A batch's groups by launch: those that do not descend and those that do where
