@@ -270,7 +270,7 @@ int gpj_batch_create(gpj_ctx *ctx, const uint8_t *d_input, uint64_t input_bytes,
   std::vector<uint32_t> slots(num_queries);
   for (uint32_t g = 0; g < num_queries; ++g) {
     const gpj_batch_query &Qg = queries[g];
-    if (Qg.h_ir == nullptr || ir_off + int(Qg.ir_len) > gpjb::kMaxQueryIrBytes ||
+    if (Qg.h_ir == nullptr || Qg.ir_len > uint64_t(gpjb::kMaxQueryIrBytes - ir_off) ||
         Qg.num_levels > uint32_t(GPJ_MAX_LEVELS) || Qg.base_level >= Qg.num_levels) {
       delete b;
       return gpjb::report_error(GPJ_ERR_INVALID_ARGUMENT,
